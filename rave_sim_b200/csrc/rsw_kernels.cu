@@ -86,6 +86,78 @@ __global__ void natural_to_spec_kernel(const Cx *__restrict__ in, Cx *__restrict
         out[spec_addr(k, v)] = in[k];
 }
 
+// digitrev_rt / digitpos_rt of indices below 2^31 in 32-bit arithmetic, RB the
+// digit width
+template <int RB> __device__ __forceinline__ int digitrev_32(int p, int log_l) {
+    int f = 0, sh = 0;
+    for (int left = log_l; left > 0; left -= RB) {  // top digit first
+        const int lr = left < RB ? left : RB;
+        f |= ((p >> (left - lr)) & ((1 << lr) - 1)) << sh;
+        sh += lr;
+    }
+    return f;
+}
+template <int RB> __device__ __forceinline__ int digitpos_32(int f, int log_l) {
+    int p = 0, sh = 0;
+    for (int left = log_l; left > 0; left -= RB) {
+        const int lr = left < RB ? left : RB;
+        p |= ((f >> sh) & ((1 << lr) - 1)) << (left - lr);
+        sh += lr;
+    }
+    return p;
+}
+__device__ __forceinline__ int digitrev_i(int p, int log_l, int rb) {
+    return rb == 3 ? digitrev_32<3>(p, log_l) : digitrev_32<4>(p, log_l);
+}
+__device__ __forceinline__ int digitpos_i(int f, int log_l, int rb) {
+    return rb == 3 ? digitpos_32<3>(f, log_l) : digitpos_32<4>(f, log_l);
+}
+
+// Spectrum layout <-> natural frequency order of multi-level plans, through
+// shared memory. A gather by spec_addr moves a whole sector per sample on one
+// side (consecutive frequencies lie a row apart). A tile of K consecutive
+// column frequencies k1 by P consecutive row positions is contiguous on both
+// sides instead: P samples of K rows in the spectrum, K samples at P places
+// (2^log_nb N1 apart, in digit-reversed order) in natural order. One read and
+// one write of the field, so the memory copy bounds it.
+template <typename Cx, bool TO_NATURAL, int LOG_K, int LOG_P>
+__global__ void __launch_bounds__(256) spec_tile_kernel(const Cx *__restrict__ in, Cx *__restrict__ out, int64_t n,
+                                                        SpecLevels v) {
+    constexpr int K = 1 << LOG_K, P = 1 << LOG_P;
+    __shared__ Cx tile[K][P + 1];
+    const int log_len = v.log_n1 + v.log_nb + v.log_nr;
+    const int log_tp = v.log_nr - LOG_P, log_tk = v.log_n1 - LOG_K;  // tiles along a row, along k1
+    const int t = threadIdx.x;
+    const int64_t tiles = n >> (LOG_K + LOG_P);
+    for (int64_t id = blockIdx.x; id < tiles; id += gridDim.x) {
+        // row positions innermost, then the middle level, then k1, then the transforms
+        const int pr0 = int(id & ((int64_t(1) << log_tp) - 1)) << LOG_P;
+        const int pb = int((id >> log_tp) & ((int64_t(1) << v.log_nb) - 1));
+        const int k10 = int((id >> (log_tp + v.log_nb)) & ((int64_t(1) << log_tk) - 1)) << LOG_K;
+        const int64_t seq = (id >> (log_tp + v.log_nb + log_tk)) << log_len;
+        const int64_t spec0 = seq + (int64_t(pb) << v.log_nr) + pr0;
+        const int64_t nat0 = seq + k10 + (int64_t(digitrev_i(pb, v.log_nb, v.rb_nb)) << v.log_n1);
+        const auto spec = [&](int i, int j) {  // k1 = k10 + i, row position pr0 + j
+            return spec0 + (int64_t(digitpos_i(k10 + i, v.log_n1, v.rb_n1)) << (v.log_nb + v.log_nr)) + j;
+        };
+        const auto natural = [&](int i, int j) {
+            return nat0 + (int64_t(digitrev_i(pr0 + j, v.log_nr, v.rb_nr)) << (v.log_nb + v.log_n1)) + i;
+        };
+#pragma unroll 8
+        for (int e = t; e < K * P; e += 256) {
+            if constexpr (TO_NATURAL) tile[e / P][e % P] = in[spec(e / P, e % P)];
+            else tile[e % K][e / K] = in[natural(e % K, e / K)];
+        }
+        __syncthreads();
+#pragma unroll 8
+        for (int e = t; e < K * P; e += 256) {
+            if constexpr (TO_NATURAL) out[natural(e % K, e / K)] = tile[e % K][e / K];
+            else out[spec(e / P, e % P)] = tile[e / P][e % P];
+        }
+        __syncthreads();
+    }
+}
+
 template <typename Cx>
 __global__ void trans_kernel(Cx *__restrict__ u, int64_t n, TransArgs tr) {
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
@@ -207,23 +279,41 @@ static unsigned grid_for(int64_t n, int threads) {
     return unsigned(b < 1 ? 1 : (b > cap ? cap : b));
 }
 
+// Runs of 512 bytes on both sides of a tile (complex64 tiles of 64 x 64,
+// complex128 32 x 32), 16-sample runs where the column level has only 16.
+template <typename Cx, bool TO_NATURAL, int LOG_K, int LOG_P>
+static void spec_tiles(const Cx *in, Cx *out, int64_t n, const SpecLevels &v, cudaStream_t s) {
+    const int64_t tiles = n >> (LOG_K + LOG_P);
+    const unsigned g = unsigned(tiles < 148 * 16 ? tiles : 148 * 16);
+    spec_tile_kernel<Cx, TO_NATURAL, LOG_K, LOG_P><<<g, 256, 0, s>>>(in, out, n, v);
+}
+// Single-level layouts (a permutation inside one row) and fields below 2^18
+// samples stay with the gather: the caches hold them, and there are too few
+// tiles to fill the device (2^15 complex128: the gather is 3 us faster).
+template <typename Cx, bool TO_NATURAL>
+static cudaError_t spec_permute(const Cx *in, Cx *out, int64_t n, const SpecLevels &v, cudaStream_t s) {
+    ++g_launches;
+    constexpr int LOG_T = sizeof(Cx) == 8 ? 6 : 5;
+    if (v.log_n1 >= 4 && v.log_nr >= LOG_T && n >= (int64_t(1) << 18)) {
+        if (v.log_n1 >= LOG_T) spec_tiles<Cx, TO_NATURAL, LOG_T, LOG_T>(in, out, n, v, s);
+        else if (v.log_n1 == 5) spec_tiles<Cx, TO_NATURAL, 5, LOG_T>(in, out, n, v, s);
+        else spec_tiles<Cx, TO_NATURAL, 4, LOG_T>(in, out, n, v, s);
+    } else if (TO_NATURAL) {
+        spec_to_natural_kernel<Cx><<<grid_for(n, 256), 256, 0, s>>>(in, out, n, v);
+    } else {
+        natural_to_spec_kernel<Cx><<<grid_for(n, 256), 256, 0, s>>>(in, out, n, v);
+    }
+    return cudaGetLastError();
+}
 cudaError_t launch_spec_to_natural(const void *in, void *out, int64_t n, const SpecLevels &v, bool dbl,
                                    cudaStream_t s) {
-    ++g_launches;
-    if (dbl)
-        spec_to_natural_kernel<double2><<<grid_for(n, 256), 256, 0, s>>>((const double2 *)in, (double2 *)out, n, v);
-    else
-        spec_to_natural_kernel<float2><<<grid_for(n, 256), 256, 0, s>>>((const float2 *)in, (float2 *)out, n, v);
-    return cudaGetLastError();
+    if (dbl) return spec_permute<double2, true>((const double2 *)in, (double2 *)out, n, v, s);
+    return spec_permute<float2, true>((const float2 *)in, (float2 *)out, n, v, s);
 }
 cudaError_t launch_natural_to_spec(const void *in, void *out, int64_t n, const SpecLevels &v, bool dbl,
                                    cudaStream_t s) {
-    ++g_launches;
-    if (dbl)
-        natural_to_spec_kernel<double2><<<grid_for(n, 256), 256, 0, s>>>((const double2 *)in, (double2 *)out, n, v);
-    else
-        natural_to_spec_kernel<float2><<<grid_for(n, 256), 256, 0, s>>>((const float2 *)in, (float2 *)out, n, v);
-    return cudaGetLastError();
+    if (dbl) return spec_permute<double2, false>((const double2 *)in, (double2 *)out, n, v, s);
+    return spec_permute<float2, false>((const float2 *)in, (float2 *)out, n, v, s);
 }
 cudaError_t launch_trans(void *u, int64_t n, const TransArgs &tr, bool dbl, cudaStream_t s) {
     ++g_launches;
