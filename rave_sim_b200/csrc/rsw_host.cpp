@@ -54,7 +54,10 @@ cudaError_t launch_blue_pre(const void *in, void *w, int64_t n, int64_t m, const
 cudaError_t launch_blue_mul(void *w, const double2 *bh, int64_t m, bool dbl, cudaStream_t s);
 cudaError_t launch_blue_post(const void *w, void *out, int64_t n, const double2 *b, double scale, bool conj_out,
                              bool dbl, cudaStream_t s);
-cudaError_t launch_prop_natural(void *U, int64_t n, const PropArgs &p, bool dbl, cudaStream_t s);
+cudaError_t launch_blue_transfer(void *w, void *U, bool given, int64_t n, int64_t m, const double2 *b,
+                                 const PropArgs &p, bool dbl, cudaStream_t s);
+cudaError_t launch_blue_table(const double2 *nat, double2 *out, int64_t m, const SpecLevels &v, int log_e,
+                              cudaStream_t s);
 unsigned long long launch_count();
 }  // namespace rsw
 
@@ -336,7 +339,8 @@ struct rsw_plan_s {
     DevBuf h3_call;                                       // per-call chirp table
     // lengths that are not a power of two (Bluestein): the power-of-two plan
     // of length m >= 2n - 1, the chirp exp(i pi k^2 / n) (n entries, FP64), the
-    // FP64 spectrum of the extended chirp (m entries) and m samples of work space
+    // FP64 spectrum of the extended chirp (m entries, in the order in which
+    // blue_convolve meets it) and m samples of work space
     bool blue = false;
     std::unique_ptr<rsw_plan_s> inner;
     int64_t m = 0;
@@ -833,6 +837,11 @@ static rsw_status launch_split_step(const rsw_plan_s *P, PassArgs a, bool mid_in
     return RSW_OK;
 }
 
+static SpecLevels spec_levels(const rsw_plan_s *p) {
+    return SpecLevels{p->log_n1, p->log_nb, p->log_nr, digit_bits(p->col_e), digit_bits(p->mid_e),
+                      digit_bits(p->row_e)};
+}
+
 // ================================================================== C ABI
 extern "C" {
 
@@ -923,22 +932,68 @@ static rsw_status create_blue_plan(rsw_plan *out, int64_t n, int dtype) {
         own.reset(p64);
     }
     CHECK(rsw_fft_forward(p64, p->bhat.p, p->bhat.p, nullptr));
-    CU(cudaDeviceSynchronize());  // the spectrum is complete before the temporary plan goes
+    CU(cudaDeviceSynchronize());  // done before its plan and scratch go (room for the second copy)
+    own.reset();
+    p->inner->scratch.release();
+    // the layout in which the convolution meets it (blue_convolve)
+    DevBuf nat = std::move(p->bhat);
+    CHECK(p->bhat.alloc(size_t(m) * sizeof(double2)));
+    const SpecLevels lv = spec_levels(p->inner.get());
+    cudaError_t e = p->inner->row_e == 16
+                        ? launch_blue_table((const double2 *)nat.p, (double2 *)p->bhat.p, m, lv, 4, nullptr)
+                        : launch_natural_to_spec(nat.p, p->bhat.p, m, lv, true, nullptr);
+    if (e != cudaSuccess) return fail(RSW_ERR_CUDA, "bluestein: %s", cudaGetErrorString(e));
+    CU(cudaDeviceSynchronize());
+    nat.release();
     CHECK(p->bwork.alloc(size_t(m) * p->elem()));
     *out = p.release();
     return RSW_OK;
 }
 
+// The circular convolution with the chirp, in place in the work space: the
+// passes of a forward and an inverse transform of length m with the chirp's
+// spectrum multiplied in between, in the internal spectrum layout (no
+// reordering), inside the row pass where its kernel exists (16 samples per
+// thread; a registered tuning may choose others).
+static rsw_status blue_convolve(rsw_plan_s *p, cudaStream_t s) {
+    const rsw_plan_s *q = p->inner.get();
+    const bool multi = q->log_n1 > 0;
+    PassArgs a = base_args(q);
+    a.in = a.out = p->bwork.p;
+    if (multi) {
+        a.flags = PF_FWD | PF_TW;
+        CHECK(run_col(q, a, s));
+        if (q->three()) CHECK(run_mid(q, a, true, s));
+    }
+    PassArgs r = row_level(q, a);
+    const int back = multi ? row_tw(q, false, true) : PF_SCALE;
+    if (q->row_e == 16) {
+        r.pr.table = (const double2 *)p->bhat.p;
+        r.flags = PF_FWD | PF_INV | row_tw(q, true, false) | back;
+        CHECK(run_row(q, r, s));
+    } else {
+        r.flags = PF_FWD | row_tw(q, true, false);
+        CHECK(run_row(q, r, s));
+        cudaError_t e = launch_blue_mul(p->bwork.p, (const double2 *)p->bhat.p, p->m, p->dbl(), s);
+        if (e != cudaSuccess) return fail(RSW_ERR_CUDA, "bluestein: %s", cudaGetErrorString(e));
+        r.flags = PF_SPEC_IN | PF_INV | back;
+        CHECK(run_row(q, r, s));
+    }
+    if (multi) {
+        if (q->three()) CHECK(run_mid(q, a, false, s));
+        a.flags = col_inv(q);
+        CHECK(run_col(q, a, s));
+    }
+    return RSW_OK;
+}
+
 // Natural-order DFT of a Bluestein plan (inverse: conj(DFT(conj X)) / n).
 static rsw_status blue_transform(rsw_plan_s *p, const void *in, void *out, bool inverse, cudaStream_t s) {
-    cudaError_t e = launch_blue_pre(in, p->bwork.p, p->n, p->m, (const double2 *)p->bchirp.p, inverse, p->dbl(), s);
+    const double2 *b = (const double2 *)p->bchirp.p;
+    cudaError_t e = launch_blue_pre(in, p->bwork.p, p->n, p->m, b, inverse, p->dbl(), s);
     if (e != cudaSuccess) return fail(RSW_ERR_CUDA, "bluestein: %s", cudaGetErrorString(e));
-    CHECK(rsw_fft_forward(p->inner.get(), p->bwork.p, p->bwork.p, s));
-    e = launch_blue_mul(p->bwork.p, (const double2 *)p->bhat.p, p->m, p->dbl(), s);
-    if (e != cudaSuccess) return fail(RSW_ERR_CUDA, "bluestein: %s", cudaGetErrorString(e));
-    CHECK(rsw_fft_inverse(p->inner.get(), p->bwork.p, p->bwork.p, s));
-    e = launch_blue_post(p->bwork.p, out, p->n, (const double2 *)p->bchirp.p, inverse ? 1.0 / double(p->n) : 1.0,
-                         inverse, p->dbl(), s);
+    CHECK(blue_convolve(p, s));
+    e = launch_blue_post(p->bwork.p, out, p->n, b, inverse ? 1.0 / double(p->n) : 1.0, inverse, p->dbl(), s);
     if (e != cudaSuccess) return fail(RSW_ERR_CUDA, "bluestein: %s", cudaGetErrorString(e));
     return RSW_OK;
 }
@@ -946,15 +1001,19 @@ static rsw_status blue_transform(rsw_plan_s *p, const void *in, void *out, bool 
 // propagate() of a Bluestein plan: U = FFT(u) (unless given), transfer
 // function and cutoff on the natural-order spectrum, u = iFFT(U).
 static rsw_status blue_propagate(rsw_plan_s *p, void *u, void *U, const PropArgs &pr, bool skip_fft, cudaStream_t s) {
-    void *spec = U;
-    if (!spec) {
-        CHECK(p->scratch.alloc(size_t(p->n) * p->elem()));
-        spec = p->scratch.p;
+    const double2 *b = (const double2 *)p->bchirp.p;
+    cudaError_t e = cudaSuccess;
+    if (!skip_fft) {
+        e = launch_blue_pre(u, p->bwork.p, p->n, p->m, b, false, p->dbl(), s);
+        if (e != cudaSuccess) return fail(RSW_ERR_CUDA, "bluestein: %s", cudaGetErrorString(e));
+        CHECK(blue_convolve(p, s));
     }
-    if (!skip_fft) CHECK(blue_transform(p, u, spec, false, s));
-    cudaError_t e = launch_prop_natural(spec, p->n, pr, p->dbl(), s);
+    e = launch_blue_transfer(p->bwork.p, U, skip_fft, p->n, p->m, b, pr, p->dbl(), s);
     if (e != cudaSuccess) return fail(RSW_ERR_CUDA, "transfer function: %s", cudaGetErrorString(e));
-    return blue_transform(p, spec, u, true, s);
+    CHECK(blue_convolve(p, s));
+    e = launch_blue_post(p->bwork.p, u, p->n, b, 1.0 / double(p->n), true, p->dbl(), s);
+    if (e != cudaSuccess) return fail(RSW_ERR_CUDA, "bluestein: %s", cudaGetErrorString(e));
+    return RSW_OK;
 }
 
 rsw_status rsw_plan_create(rsw_plan *out, int64_t n, int dtype) {
@@ -1137,10 +1196,6 @@ rsw_status rsw_plan_set_propagator(rsw_plan p, int mode) {
 
 static rsw_status need_scratch(rsw_plan_s *p) { return p->scratch.alloc(size_t(p->n) * p->elem()); }
 
-static SpecLevels spec_levels(const rsw_plan_s *p) {
-    return SpecLevels{p->log_n1, p->log_nb, p->log_nr, digit_bits(p->col_e), digit_bits(p->mid_e),
-                      digit_bits(p->row_e)};
-}
 static cudaError_t to_natural(const rsw_plan_s *p, const void *spec, void *nat, cudaStream_t s) {
     return launch_spec_to_natural(spec, nat, p->n, spec_levels(p), p->dbl(), s);
 }

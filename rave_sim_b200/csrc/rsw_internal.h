@@ -61,6 +61,10 @@ struct PropArgs {
     // per sample (no chirp form); evanescent fx^2 >= inv_wl2 is zeroed.
     int exact;
     double inv_wl, inv_wl2, z2pi;
+    // Convolution plans (lengths that are not a power of two): the spectrum is
+    // multiplied by this FP64 table instead, entry (row, r, tp) at
+    // row * L + r * T + tp (the row kernel's register order: coalesced)
+    const double2 *table;
 };
 
 enum PassFlags : int {

@@ -378,15 +378,13 @@ unsigned long long launch_count() { return g_launches.load(); }
 //   X[k] = conj(b[k]) sum_j (x[j] conj(b[j])) b[k - j].
 // The pointwise products are taken in FP64 for both field types (the tables
 // are FP64), so the fields round once per product.
-__device__ __forceinline__ double2 to_d(double2 a) { return a; }
-__device__ __forceinline__ double2 to_d(float2 a) { return make_double2(double(a.x), double(a.y)); }
 template <typename Cx>
 __global__ void blue_pre_kernel(const Cx *__restrict__ in, Cx *__restrict__ w, int64_t n, int64_t m,
                                 const double2 *__restrict__ b, int conj_in) {
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < m; k += stride) {
         if (k < n) {
-            double2 x = to_d(in[k]);
+            double2 x = to_f64(in[k]);
             if (conj_in) x.y = -x.y;
             w[k] = to_c(cmulc(x, b[k]), Cx{});
         } else {
@@ -398,49 +396,76 @@ template <typename Cx>
 __global__ void blue_mul_kernel(Cx *__restrict__ w, const double2 *__restrict__ bh, int64_t m) {
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < m; k += stride)
-        w[k] = to_c(cmul(to_d(w[k]), bh[k]), Cx{});
+        w[k] = to_c(cmul(to_f64(w[k]), bh[k]), Cx{});
 }
 template <typename Cx>
 __global__ void blue_post_kernel(const Cx *__restrict__ w, Cx *__restrict__ out, int64_t n,
                                  const double2 *__restrict__ b, double scale, int conj_out) {
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < n; k += stride) {
-        double2 y = cmulc(to_d(w[k]), b[k]);
+        double2 y = cmulc(to_f64(w[k]), b[k]);
         y = make_double2(y.x * scale, (conj_out ? -y.y : y.y) * scale);
         out[k] = to_c(y, Cx{});
     }
 }
+// The chirp's spectrum (natural order, length m) in the row kernel's register
+// order (PropArgs::table): entry (row, r, tp) of rows of 2^log_nr with e
+// samples per thread
+__global__ void blue_table_kernel(const double2 *__restrict__ nat, double2 *__restrict__ out, int64_t m, SpecLevels v,
+                                  int log_e) {
+    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+    const int log_t = v.log_nr - log_e;
+    const int lrl = stage_lr(v.log_nr, stage_count(v.log_nr, v.rb_nr) - 1, v.rb_nr);  // last radix
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < m; i += stride) {
+        const int r = int(i >> log_t) & ((1 << log_e) - 1), tp = int(i) & ((1 << log_t) - 1);
+        const int64_t row = i >> v.log_nr;
+        int q = 0;  // bit-reversed digit of the last stage (Block::last_off)
+        for (int bit = 0; bit < lrl; ++bit) q |= ((r >> bit) & 1) << (lrl - 1 - bit);
+        const int pr = (tp << log_e) + (r >> lrl << lrl) + q;
+        const int64_t k1 = digitrev_rt(row >> v.log_nb, v.log_n1, v.rb_n1);
+        const int64_t kb = digitrev_rt(row & ((int64_t(1) << v.log_nb) - 1), v.log_nb, v.rb_nb);
+        out[i] = nat[k1 + ((kb + (digitrev_rt(pr, v.log_nr, v.rb_nr) << v.log_nb)) << v.log_n1)];
+    }
+}
 // Transfer function and cutoff on a natural-order spectrum of any length:
 // ks = k or k - N (np.fft.fftfreq's order), fx = (ks * (1/N)) / dx in the
-// reference's order (big-wave/propagation.py:154-175, :124-128), applied in FP64.
+// reference's order (big-wave/propagation.py:154-175, :124-128), in FP64.
+__device__ __forceinline__ double2 natural_transfer(const PropArgs &p, int64_t k, int64_t n, double2 X) {
+    if (p.has_cut && k >= p.cut_lo && k < p.cut_hi) return make_double2(0.0, 0.0);
+    if (!p.has_h) return X;
+    const int64_t ks = k < (n - 1) / 2 + 1 ? k : k - n;
+    const double fx = __ddiv_rn(__dmul_rn(double(ks), p.fac), p.dx);
+    double ph;
+    if (p.exact) {
+        const double f2 = __dmul_rn(fx, fx);
+        const double d = __dsub_rn(p.inv_wl2, f2);
+        if (!(d > 0.0)) return make_double2(0.0, 0.0);
+        ph = __ddiv_rn(__dmul_rn(p.z2pi, f2), __dadd_rn(p.inv_wl, __dsqrt_rn(d)));
+    } else {
+        ph = __dmul_rn(p.c, __dmul_rn(fx, fx));
+    }
+    double sn, cs;
+    sincos_phase(ph, &sn, &cs);
+    return cmul(X, make_double2(p.A.x * cs - p.A.y * sn, p.A.x * sn + p.A.y * cs));
+}
+// Between the two transforms of propagate: the spectrum X[k] = conj(b[k])
+// w[k] (or the given one, U), times the transfer function, and the
+// premultiplied input of the inverse transform, conj(X H) conj(b[k]), zero
+// from n to m; U receives X H where it is wanted. One sweep in place of a
+// post-multiplication, a product and a pre-multiplication.
 template <typename Cx>
-__global__ void prop_natural_kernel(Cx *__restrict__ U, int64_t n, PropArgs p) {
+__global__ void blue_transfer_kernel(Cx *__restrict__ w, Cx *__restrict__ U, int given, int64_t n, int64_t m,
+                                     const double2 *__restrict__ b, PropArgs p) {
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    const int64_t pos_end = (n - 1) / 2 + 1;
-    for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < n; k += stride) {
-        if (p.has_cut && k >= p.cut_lo && k < p.cut_hi) {
-            U[k] = to_c(make_double2(0.0, 0.0), Cx{});
-            continue;
+    for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < m; k += stride) {
+        double2 y = make_double2(0.0, 0.0);
+        if (k < n) {
+            const double2 bk = b[k];
+            const double2 X = natural_transfer(p, k, n, given ? to_f64(U[k]) : cmulc(to_f64(w[k]), bk));
+            if (U) U[k] = to_c(X, Cx{});
+            y = cmulc(make_double2(X.x, -X.y), bk);
         }
-        if (!p.has_h) continue;
-        const int64_t ks = k < pos_end ? k : k - n;
-        const double fx = __ddiv_rn(__dmul_rn(double(ks), p.fac), p.dx);
-        double ph;
-        if (p.exact) {
-            const double f2 = __dmul_rn(fx, fx);
-            const double d = __dsub_rn(p.inv_wl2, f2);
-            if (!(d > 0.0)) {
-                U[k] = to_c(make_double2(0.0, 0.0), Cx{});
-                continue;
-            }
-            ph = __ddiv_rn(__dmul_rn(p.z2pi, f2), __dadd_rn(p.inv_wl, __dsqrt_rn(d)));
-        } else {
-            ph = __dmul_rn(p.c, __dmul_rn(fx, fx));
-        }
-        double sn, cs;
-        sincos_phase(ph, &sn, &cs);
-        const double2 H = make_double2(p.A.x * cs - p.A.y * sn, p.A.x * sn + p.A.y * cs);
-        U[k] = to_c(cmul(to_d(U[k]), H), Cx{});
+        w[k] = to_c(y, Cx{});
     }
 }
 
@@ -470,10 +495,18 @@ cudaError_t launch_blue_post(const void *w, void *out, int64_t n, const double2 
                                                                  conj_out);
     return cudaGetLastError();
 }
-cudaError_t launch_prop_natural(void *U, int64_t n, const PropArgs &p, bool dbl, cudaStream_t s) {
+cudaError_t launch_blue_transfer(void *w, void *U, bool given, int64_t n, int64_t m, const double2 *b,
+                                 const PropArgs &p, bool dbl, cudaStream_t s) {
     ++g_launches;
-    if (dbl) prop_natural_kernel<double2><<<grid_for(n, 256), 256, 0, s>>>((double2 *)U, n, p);
-    else prop_natural_kernel<float2><<<grid_for(n, 256), 256, 0, s>>>((float2 *)U, n, p);
+    if (dbl)
+        blue_transfer_kernel<double2><<<grid_for(m, 256), 256, 0, s>>>((double2 *)w, (double2 *)U, given, n, m, b, p);
+    else blue_transfer_kernel<float2><<<grid_for(m, 256), 256, 0, s>>>((float2 *)w, (float2 *)U, given, n, m, b, p);
+    return cudaGetLastError();
+}
+cudaError_t launch_blue_table(const double2 *nat, double2 *out, int64_t m, const SpecLevels &v, int log_e,
+                              cudaStream_t s) {
+    ++g_launches;
+    blue_table_kernel<<<grid_for(m, 256), 256, 0, s>>>(nat, out, m, v, log_e);
     return cudaGetLastError();
 }
 

@@ -363,6 +363,9 @@ template <> __device__ __forceinline__ float2 one_c<float2>() { return make_floa
 __device__ __forceinline__ double2 cvt(double2 a, double2) { return a; }
 __device__ __forceinline__ float2 cvt(double2 a, float2) { return make_float2(float(a.x), float(a.y)); }
 
+__device__ __forceinline__ double2 to_f64(double2 a) { return a; }
+__device__ __forceinline__ double2 to_f64(float2 a) { return make_double2(double(a.x), double(a.y)); }
+
 // W_N^m from the FP64 four-step tables (lo[m & mask] * hi[m >> shift]).
 __device__ __forceinline__ double2 w4(const PassArgs &a, int64_t m) {
     const double2 *lo = static_cast<const double2 *>(a.tw4_lo);
@@ -626,6 +629,10 @@ __global__ void __launch_bounds__(Block<Real, LOG_L2, 1, E>::NT, row_min_ctas<Re
                     if (unsigned((fbase | B::freq_off(r)) - k2lo) < cut_span) v[r] = Cx{};
             }
           }
+        } else if (a.pr.table) {
+            const double2 *tab = a.pr.table + (row << LOG_L2) + tp;
+#pragma unroll
+            for (int r = 0; r < E; ++r) v[r] = cvt(cmul(to_f64(v[r]), __ldg(tab + r * B::T)), Cx{});
         } else if (a.pr.has_h || a.pr.has_cut) {
             const int64_t half2 = int64_t(1) << (LOG_L2 - 1);
 #pragma unroll
