@@ -408,17 +408,28 @@ template <int T> struct ColTab {
 // row (tile) are factored into 64 + len/64 entries built once per row (tile).
 // CHIRP: transfer function in the factored chirp form (two-level plans), else
 // the per-sample formula (single-level plans).
-// Complex64 rows of 2^13 (512 threads) run two CTAs per SM at 64 registers:
-// 8 % faster than one CTA at 121 registers.
-template <typename Real, int LOG_L2, int E> constexpr int row_min_ctas() {
-    return sizeof(Real) == 4 && LOG_L2 == 13 && E == 16 ? 2 : 1;
+// Registers of long rows are capped by the threads an SM should hold: left
+// alone, ptxas gave the row kernels of 128 to 256 threads 230 to 250
+// registers, which left 8 warps on an SM. complex128 rows of 2^12 run 16 warps
+// at 128 registers (16 samples per thread; 8 per thread: 32 warps at 64),
+// complex64 rows from 2^11 32 warps at 64. One split step over 8 fields of
+// 2^22 (best split): complex128 25.0 -> 23.6 ps per sample, complex64 15.1 ->
+// 14.0; 24 warps at 80 registers: 24.3 and 14.0. Rows of 2^13 and more fill
+// the SM at these counts anyway. Shorter rows stay uncapped: the caps made
+// them spill in the factor tables' sincospi (complex128 2^10 2 %, 2^8 7 % and
+// 2^11 forward rows 10 % slower). So do single rows (no chirp form).
+template <typename Real, int LOG_L2, int E, bool CHIRP> constexpr int row_min_ctas() {
+    if (E == 32 || LOG_L2 < (sizeof(Real) == 8 && E == 16 ? 12 : 11)) return 1;
+    if (!CHIRP && !(sizeof(Real) == 4 && LOG_L2 == 13)) return 1;
+    constexpr int want = (sizeof(Real) == 8 && E == 16 ? 512 : 1024) / ((1 << LOG_L2) / E);
+    return want < 1 ? 1 : want;
 }
 // TWF: the three-level variant with the W_{N2} twiddle before the forward
 // transform (a separate kernel, so that the two-level one carries no code for it).
 // BATCH: the batched variant (per-instance transfer functions, a.bpr; chirp
 // form only), also a separate kernel so that the others carry no code for it.
 template <typename Real, int LOG_L2, int E, bool CHIRP, bool TWF = false, bool BATCH = false>
-__global__ void __launch_bounds__(Block<Real, LOG_L2, 1, E>::NT, row_min_ctas<Real, LOG_L2, E>()) row_pass_kernel(PassArgs a) {
+__global__ void __launch_bounds__(Block<Real, LOG_L2, 1, E>::NT, row_min_ctas<Real, LOG_L2, E, CHIRP>()) row_pass_kernel(PassArgs a) {
     using B = Block<Real, LOG_L2, 1, E>;
     using Cx = typename B::Cx;
     constexpr int L = B::L;
