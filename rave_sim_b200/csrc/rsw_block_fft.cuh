@@ -496,10 +496,17 @@ struct Block : Radix<LOG_L, E_, direct_max_ls(2 * sizeof(Real), LOG_L)> {
     __device__ static __forceinline__ int freq_base(int tp) { return digitrev_c(tp * E, LOG_L, Rx::RB); }
     __device__ static __forceinline__ int last_freq(int tp, int r) { return freq_base(tp) | freq_off(r); }
 
-    // copy the block's twiddle tables (global, host-built layout) into shared memory
-    __device__ static __forceinline__ void load_twiddles(Tw *tw_sm, const Tw *__restrict__ tw_g) {
-        for (int k = threadIdx.x; k < Rx::TW; k += NT) tw_sm[k] = tw_g[k];
+    // copy the block's twiddle tables (global, host-built layout) into shared
+    // memory, asynchronously: every thread's copies are in flight at once;
+    // twiddles_loaded() and a barrier complete them
+    __device__ static __forceinline__ void load_twiddles(Tw *tw_sm, const Tw *tw_g) {
+        const unsigned dst = unsigned(__cvta_generic_to_shared(tw_sm));
+        for (int k = threadIdx.x; k < Rx::TW; k += NT)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst + unsigned(k * sizeof(Tw))),
+                         "l"(tw_g + k), "n"(sizeof(Tw))
+                         : "memory");
     }
+    __device__ static __forceinline__ void twiddles_loaded() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 };
 
 }  // namespace rsw

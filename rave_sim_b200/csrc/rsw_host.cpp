@@ -56,8 +56,6 @@ cudaError_t launch_blue_post(const void *w, void *out, int64_t n, const double2 
                              bool dbl, cudaStream_t s);
 cudaError_t launch_blue_transfer(void *w, void *U, bool given, int64_t n, int64_t m, const double2 *b,
                                  const PropArgs &p, bool dbl, cudaStream_t s);
-cudaError_t launch_blue_table(const double2 *nat, double2 *out, int64_t m, const SpecLevels &v, int log_e,
-                              cudaStream_t s);
 unsigned long long launch_count();
 }  // namespace rsw
 
@@ -339,8 +337,8 @@ struct rsw_plan_s {
     DevBuf h3_call;                                       // per-call chirp table
     // lengths that are not a power of two (Bluestein): the power-of-two plan
     // of length m >= 2n - 1, the chirp exp(i pi k^2 / n) (n entries, FP64), the
-    // FP64 spectrum of the extended chirp (m entries, in the order in which
-    // blue_convolve meets it) and m samples of work space
+    // FP64 spectrum of the extended chirp (m entries, in the inner plan's
+    // spectrum layout) and m samples of work space
     bool blue = false;
     std::unique_ptr<rsw_plan_s> inner;
     int64_t m = 0;
@@ -838,8 +836,9 @@ static rsw_status launch_split_step(const rsw_plan_s *P, PassArgs a, bool mid_in
 }
 
 static SpecLevels spec_levels(const rsw_plan_s *p) {
+    const int log_e = p->row_e == 8 ? 3 : p->row_e == 16 ? 4 : 5;
     return SpecLevels{p->log_n1, p->log_nb, p->log_nr, digit_bits(p->col_e), digit_bits(p->mid_e),
-                      digit_bits(p->row_e)};
+                      digit_bits(p->row_e), log_e};
 }
 
 // ================================================================== C ABI
@@ -935,13 +934,9 @@ static rsw_status create_blue_plan(rsw_plan *out, int64_t n, int dtype) {
     CU(cudaDeviceSynchronize());  // done before its plan and scratch go (room for the second copy)
     own.reset();
     p->inner->scratch.release();
-    // the layout in which the convolution meets it (blue_convolve)
     DevBuf nat = std::move(p->bhat);
     CHECK(p->bhat.alloc(size_t(m) * sizeof(double2)));
-    const SpecLevels lv = spec_levels(p->inner.get());
-    cudaError_t e = p->inner->row_e == 16
-                        ? launch_blue_table((const double2 *)nat.p, (double2 *)p->bhat.p, m, lv, 4, nullptr)
-                        : launch_natural_to_spec(nat.p, p->bhat.p, m, lv, true, nullptr);
+    cudaError_t e = launch_natural_to_spec(nat.p, p->bhat.p, m, spec_levels(p->inner.get()), true, nullptr);
     if (e != cudaSuccess) return fail(RSW_ERR_CUDA, "bluestein: %s", cudaGetErrorString(e));
     CU(cudaDeviceSynchronize());
     nat.release();

@@ -62,8 +62,7 @@ struct PropArgs {
     int exact;
     double inv_wl, inv_wl2, z2pi;
     // Convolution plans (lengths that are not a power of two): the spectrum is
-    // multiplied by this FP64 table instead, entry (row, r, tp) at
-    // row * L + r * T + tp (the row kernel's register order: coalesced)
+    // multiplied by this FP64 table instead, in the spectrum layout (SpecLevels)
     const double2 *table;
 };
 
@@ -159,6 +158,9 @@ struct PassArgs {
     // column pass: when set, the launch functions store the kernel's resident
     // CTAs on the current device here and launch nothing
     int64_t *resident;
+    // launch after the preceding kernel has completed: its tables were written
+    // in this stream (programmatic dependent launch reads them before)
+    int serial;
     // column pass, filled in by its launch function: a 2-D TMA map over the
     // input (rows of 2^log_n2 samples as 8-byte words; boxes of one tile's
     // columns by up to 256 rows), through which each CTA prefetches its next
@@ -168,10 +170,15 @@ struct PassArgs {
 };
 
 // Level structure of the internal spectrum layout (log2 lengths and digit
-// widths of the column, middle and row levels).
+// widths of the column, middle and row levels). Within a row the samples lie
+// in the row kernel's register order: register r of thread tp at r * T + tp,
+// T = 2^(log_nr - log_e) threads, so that the kernel stores and loads them
+// coalesced (its block position tp * E + ... would scatter a warp's samples
+// over 32 sectors).
 struct SpecLevels {
     int log_n1, log_nb, log_nr;
     int rb_n1, rb_nb, rb_nr;
+    int log_e;
 };
 
 // Phase-step signal retrieval: the 3 x K pseudo-inverse of [sin phi_k,

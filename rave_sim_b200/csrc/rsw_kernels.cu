@@ -59,32 +59,9 @@ cudaError_t launch_row_pass(const PassArgs &a, bool dbl, int e, cudaStream_t s) 
 
 // ---------------------------------------------------------- small kernels
 // internal spectrum layout <-> natural frequency order. Frequency
-// k = k1 + N1 (kb + Nb kr) sits at ((p1 Nb + pb) Nr + pr), p = digitpos of
-// each level's index (log_nb = 0 for two-level and single-level plans).
-// Position in the spectrum layout of natural frequency k; indices at and
-// above one transform's length address consecutive transforms (batches).
-__device__ __forceinline__ int64_t spec_addr(int64_t k, const SpecLevels &v) {
-    const int log_len = v.log_n1 + v.log_nb + v.log_nr;
-    const int64_t seq = k >> log_len << log_len;
-    const int64_t k1 = k & ((int64_t(1) << v.log_n1) - 1);
-    const int64_t kb = (k >> v.log_n1) & ((int64_t(1) << v.log_nb) - 1);
-    const int64_t kr = (k >> (v.log_n1 + v.log_nb)) & ((int64_t(1) << v.log_nr) - 1);
-    return seq + ((((digitpos_rt(k1, v.log_n1, v.rb_n1) << v.log_nb) + digitpos_rt(kb, v.log_nb, v.rb_nb))
-                   << v.log_nr) +
-                  digitpos_rt(kr, v.log_nr, v.rb_nr));
-}
-template <typename Cx>
-__global__ void spec_to_natural_kernel(const Cx *__restrict__ in, Cx *__restrict__ out, int64_t n, SpecLevels v) {
-    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < n; k += stride)
-        out[k] = in[spec_addr(k, v)];
-}
-template <typename Cx>
-__global__ void natural_to_spec_kernel(const Cx *__restrict__ in, Cx *__restrict__ out, int64_t n, SpecLevels v) {
-    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < n; k += stride)
-        out[spec_addr(k, v)] = in[k];
-}
+// k = k1 + N1 (kb + Nb kr) sits in row p1 Nb + pb, p1 and pb the digit
+// positions of k1 and kb (log_nb = 0 for two-level and single-level plans), at
+// the place of kr in the row kernel's register order (SpecLevels).
 
 // digitrev_rt / digitpos_rt of indices below 2^31 in 32-bit arithmetic, RB the
 // digit width
@@ -112,19 +89,64 @@ __device__ __forceinline__ int digitrev_i(int p, int log_l, int rb) {
 __device__ __forceinline__ int digitpos_i(int f, int log_l, int rb) {
     return rb == 3 ? digitpos_32<3>(f, log_l) : digitpos_32<4>(f, log_l);
 }
+// a thread's register number <-> offset among its E block positions
+// (Block::last_off, its own inverse): the low lrl bits reversed, lrl the log2
+// of the last stage's radix
+__device__ __forceinline__ int last_off_i(int r, const SpecLevels &v) {
+    const int lrl = v.log_nr - (v.log_nr - 1) / v.rb_nr * v.rb_nr;
+    return (r >> lrl << lrl) + int(__brev(unsigned(r) & ((1u << lrl) - 1u)) >> (32 - lrl));
+}
+// place in the row <-> frequency kr
+__device__ __forceinline__ int row_freq(int pos, const SpecLevels &v) {
+    const int log_t = v.log_nr - v.log_e;
+    return digitrev_i(((pos & ((1 << log_t) - 1)) << v.log_e) + last_off_i(pos >> log_t, v), v.log_nr, v.rb_nr);
+}
+__device__ __forceinline__ int row_place(int kr, const SpecLevels &v) {
+    const int p = digitpos_i(kr, v.log_nr, v.rb_nr);
+    return (last_off_i(p & ((1 << v.log_e) - 1), v) << (v.log_nr - v.log_e)) + (p >> v.log_e);
+}
+// Position in the spectrum layout of natural frequency k; indices at and
+// above one transform's length address consecutive transforms (batches).
+__device__ __forceinline__ int64_t spec_addr(int64_t k, const SpecLevels &v) {
+    const int log_len = v.log_n1 + v.log_nb + v.log_nr;
+    const int64_t seq = k >> log_len << log_len;
+    const int k1 = int(k & ((int64_t(1) << v.log_n1) - 1));
+    const int kb = int((k >> v.log_n1) & ((int64_t(1) << v.log_nb) - 1));
+    const int kr = int((k >> (v.log_n1 + v.log_nb)) & ((int64_t(1) << v.log_nr) - 1));
+    const int64_t row = (int64_t(digitpos_i(k1, v.log_n1, v.rb_n1)) << v.log_nb) + digitpos_i(kb, v.log_nb, v.rb_nb);
+    return seq + (row << v.log_nr) + row_place(kr, v);
+}
+template <typename Cx>
+__global__ void spec_to_natural_kernel(const Cx *__restrict__ in, Cx *__restrict__ out, int64_t n, SpecLevels v) {
+    pass_wait();
+    pass_release();
+    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+    for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < n; k += stride)
+        out[k] = __ldcg(in + spec_addr(k, v));
+}
+template <typename Cx>
+__global__ void natural_to_spec_kernel(const Cx *__restrict__ in, Cx *__restrict__ out, int64_t n, SpecLevels v) {
+    pass_wait();
+    pass_release();
+    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+    for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < n; k += stride)
+        out[spec_addr(k, v)] = __ldcg(in + k);
+}
 
 // Spectrum layout <-> natural frequency order of multi-level plans, through
 // shared memory. A gather by spec_addr moves a whole sector per sample on one
 // side (consecutive frequencies lie a row apart). A tile of K consecutive
 // column frequencies k1 by P consecutive row positions is contiguous on both
 // sides instead: P samples of K rows in the spectrum, K samples at P places
-// (2^log_nb N1 apart, in digit-reversed order) in natural order. One read and
+// (multiples of 2^log_nb N1) in natural order. One read and
 // one write of the field, so the memory copy bounds it.
 template <typename Cx, bool TO_NATURAL, int LOG_K, int LOG_P>
 __global__ void __launch_bounds__(256) spec_tile_kernel(const Cx *__restrict__ in, Cx *__restrict__ out, int64_t n,
                                                         SpecLevels v) {
     constexpr int K = 1 << LOG_K, P = 1 << LOG_P;
     __shared__ Cx tile[K][P + 1];
+    pass_wait();
+    pass_release();
     const int log_len = v.log_n1 + v.log_nb + v.log_nr;
     const int log_tp = v.log_nr - LOG_P, log_tk = v.log_n1 - LOG_K;  // tiles along a row, along k1
     const int t = threadIdx.x;
@@ -141,12 +163,12 @@ __global__ void __launch_bounds__(256) spec_tile_kernel(const Cx *__restrict__ i
             return spec0 + (int64_t(digitpos_i(k10 + i, v.log_n1, v.rb_n1)) << (v.log_nb + v.log_nr)) + j;
         };
         const auto natural = [&](int i, int j) {
-            return nat0 + (int64_t(digitrev_i(pr0 + j, v.log_nr, v.rb_nr)) << (v.log_nb + v.log_n1)) + i;
+            return nat0 + (int64_t(row_freq(pr0 + j, v)) << (v.log_nb + v.log_n1)) + i;
         };
 #pragma unroll 8
         for (int e = t; e < K * P; e += 256) {
-            if constexpr (TO_NATURAL) tile[e / P][e % P] = in[spec(e / P, e % P)];
-            else tile[e % K][e / K] = in[natural(e % K, e / K)];
+            if constexpr (TO_NATURAL) tile[e / P][e % P] = __ldcg(in + spec(e / P, e % P));
+            else tile[e % K][e / K] = __ldcg(in + natural(e % K, e / K));
         }
         __syncthreads();
 #pragma unroll 8
@@ -282,28 +304,24 @@ static unsigned grid_for(int64_t n, int threads) {
 // Runs of 512 bytes on both sides of a tile (complex64 tiles of 64 x 64,
 // complex128 32 x 32), 16-sample runs where the column level has only 16.
 template <typename Cx, bool TO_NATURAL, int LOG_K, int LOG_P>
-static void spec_tiles(const Cx *in, Cx *out, int64_t n, const SpecLevels &v, cudaStream_t s) {
+static cudaError_t spec_tiles(const Cx *in, Cx *out, int64_t n, const SpecLevels &v, cudaStream_t s) {
     const int64_t tiles = n >> (LOG_K + LOG_P);
     const unsigned g = unsigned(tiles < 148 * 16 ? tiles : 148 * 16);
-    spec_tile_kernel<Cx, TO_NATURAL, LOG_K, LOG_P><<<g, 256, 0, s>>>(in, out, n, v);
+    return launch_dependent(spec_tile_kernel<Cx, TO_NATURAL, LOG_K, LOG_P>, g, 256, 0, s, false, in, out, n, v);
 }
 // Single-level layouts (a permutation inside one row) and fields below 2^18
 // samples stay with the gather: the caches hold them, and there are too few
 // tiles to fill the device (2^15 complex128: the gather is 3 us faster).
 template <typename Cx, bool TO_NATURAL>
 static cudaError_t spec_permute(const Cx *in, Cx *out, int64_t n, const SpecLevels &v, cudaStream_t s) {
-    ++g_launches;
     constexpr int LOG_T = sizeof(Cx) == 8 ? 6 : 5;
     if (v.log_n1 >= 4 && v.log_nr >= LOG_T && n >= (int64_t(1) << 18)) {
-        if (v.log_n1 >= LOG_T) spec_tiles<Cx, TO_NATURAL, LOG_T, LOG_T>(in, out, n, v, s);
-        else if (v.log_n1 == 5) spec_tiles<Cx, TO_NATURAL, 5, LOG_T>(in, out, n, v, s);
-        else spec_tiles<Cx, TO_NATURAL, 4, LOG_T>(in, out, n, v, s);
-    } else if (TO_NATURAL) {
-        spec_to_natural_kernel<Cx><<<grid_for(n, 256), 256, 0, s>>>(in, out, n, v);
-    } else {
-        natural_to_spec_kernel<Cx><<<grid_for(n, 256), 256, 0, s>>>(in, out, n, v);
+        if (v.log_n1 >= LOG_T) return spec_tiles<Cx, TO_NATURAL, LOG_T, LOG_T>(in, out, n, v, s);
+        if (v.log_n1 == 5) return spec_tiles<Cx, TO_NATURAL, 5, LOG_T>(in, out, n, v, s);
+        return spec_tiles<Cx, TO_NATURAL, 4, LOG_T>(in, out, n, v, s);
     }
-    return cudaGetLastError();
+    return launch_dependent(TO_NATURAL ? spec_to_natural_kernel<Cx> : natural_to_spec_kernel<Cx>, grid_for(n, 256), 256,
+                            0, s, false, in, out, n, v);
 }
 cudaError_t launch_spec_to_natural(const void *in, void *out, int64_t n, const SpecLevels &v, bool dbl,
                                    cudaStream_t s) {
@@ -381,10 +399,12 @@ unsigned long long launch_count() { return g_launches.load(); }
 template <typename Cx>
 __global__ void blue_pre_kernel(const Cx *__restrict__ in, Cx *__restrict__ w, int64_t n, int64_t m,
                                 const double2 *__restrict__ b, int conj_in) {
+    pass_wait();
+    pass_release();
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < m; k += stride) {
         if (k < n) {
-            double2 x = to_f64(in[k]);
+            double2 x = to_f64(__ldcg(in + k));
             if (conj_in) x.y = -x.y;
             w[k] = to_c(cmulc(x, b[k]), Cx{});
         } else {
@@ -394,37 +414,22 @@ __global__ void blue_pre_kernel(const Cx *__restrict__ in, Cx *__restrict__ w, i
 }
 template <typename Cx>
 __global__ void blue_mul_kernel(Cx *__restrict__ w, const double2 *__restrict__ bh, int64_t m) {
+    pass_wait();
+    pass_release();
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < m; k += stride)
-        w[k] = to_c(cmul(to_f64(w[k]), bh[k]), Cx{});
+        w[k] = to_c(cmul(to_f64(__ldcg(w + k)), bh[k]), Cx{});
 }
 template <typename Cx>
 __global__ void blue_post_kernel(const Cx *__restrict__ w, Cx *__restrict__ out, int64_t n,
                                  const double2 *__restrict__ b, double scale, int conj_out) {
+    pass_wait();
+    pass_release();
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < n; k += stride) {
-        double2 y = cmulc(to_f64(w[k]), b[k]);
+        double2 y = cmulc(to_f64(__ldcg(w + k)), b[k]);
         y = make_double2(y.x * scale, (conj_out ? -y.y : y.y) * scale);
         out[k] = to_c(y, Cx{});
-    }
-}
-// The chirp's spectrum (natural order, length m) in the row kernel's register
-// order (PropArgs::table): entry (row, r, tp) of rows of 2^log_nr with e
-// samples per thread
-__global__ void blue_table_kernel(const double2 *__restrict__ nat, double2 *__restrict__ out, int64_t m, SpecLevels v,
-                                  int log_e) {
-    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    const int log_t = v.log_nr - log_e;
-    const int lrl = stage_lr(v.log_nr, stage_count(v.log_nr, v.rb_nr) - 1, v.rb_nr);  // last radix
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < m; i += stride) {
-        const int r = int(i >> log_t) & ((1 << log_e) - 1), tp = int(i) & ((1 << log_t) - 1);
-        const int64_t row = i >> v.log_nr;
-        int q = 0;  // bit-reversed digit of the last stage (Block::last_off)
-        for (int bit = 0; bit < lrl; ++bit) q |= ((r >> bit) & 1) << (lrl - 1 - bit);
-        const int pr = (tp << log_e) + (r >> lrl << lrl) + q;
-        const int64_t k1 = digitrev_rt(row >> v.log_nb, v.log_n1, v.rb_n1);
-        const int64_t kb = digitrev_rt(row & ((int64_t(1) << v.log_nb) - 1), v.log_nb, v.rb_nb);
-        out[i] = nat[k1 + ((kb + (digitrev_rt(pr, v.log_nr, v.rb_nr) << v.log_nb)) << v.log_n1)];
     }
 }
 // Transfer function and cutoff on a natural-order spectrum of any length:
@@ -456,12 +461,14 @@ __device__ __forceinline__ double2 natural_transfer(const PropArgs &p, int64_t k
 template <typename Cx>
 __global__ void blue_transfer_kernel(Cx *__restrict__ w, Cx *__restrict__ U, int given, int64_t n, int64_t m,
                                      const double2 *__restrict__ b, PropArgs p) {
+    pass_wait();
+    pass_release();
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < m; k += stride) {
         double2 y = make_double2(0.0, 0.0);
         if (k < n) {
             const double2 bk = b[k];
-            const double2 X = natural_transfer(p, k, n, given ? to_f64(U[k]) : cmulc(to_f64(w[k]), bk));
+            const double2 X = natural_transfer(p, k, n, given ? to_f64(__ldcg(U + k)) : cmulc(to_f64(__ldcg(w + k)), bk));
             if (U) U[k] = to_c(X, Cx{});
             y = cmulc(make_double2(X.x, -X.y), bk);
         }
@@ -469,47 +476,40 @@ __global__ void blue_transfer_kernel(Cx *__restrict__ w, Cx *__restrict__ U, int
     }
 }
 
+template <typename Cx> static const Cx *in_c(const void *p) { return static_cast<const Cx *>(p); }
+template <typename Cx> static Cx *out_c(void *p) { return static_cast<Cx *>(p); }
 cudaError_t launch_blue_pre(const void *in, void *w, int64_t n, int64_t m, const double2 *b, bool conj_in, bool dbl,
                             cudaStream_t s) {
-    ++g_launches;
+    const int cj = conj_in;
     if (dbl)
-        blue_pre_kernel<double2><<<grid_for(m, 256), 256, 0, s>>>((const double2 *)in, (double2 *)w, n, m, b, conj_in);
-    else
-        blue_pre_kernel<float2><<<grid_for(m, 256), 256, 0, s>>>((const float2 *)in, (float2 *)w, n, m, b, conj_in);
-    return cudaGetLastError();
+        return launch_dependent(blue_pre_kernel<double2>, grid_for(m, 256), 256, 0, s, false, in_c<double2>(in),
+                                out_c<double2>(w), n, m, b, cj);
+    return launch_dependent(blue_pre_kernel<float2>, grid_for(m, 256), 256, 0, s, false, in_c<float2>(in),
+                            out_c<float2>(w), n, m, b, cj);
 }
 cudaError_t launch_blue_mul(void *w, const double2 *bh, int64_t m, bool dbl, cudaStream_t s) {
-    ++g_launches;
-    if (dbl) blue_mul_kernel<double2><<<grid_for(m, 256), 256, 0, s>>>((double2 *)w, bh, m);
-    else blue_mul_kernel<float2><<<grid_for(m, 256), 256, 0, s>>>((float2 *)w, bh, m);
-    return cudaGetLastError();
+    if (dbl)
+        return launch_dependent(blue_mul_kernel<double2>, grid_for(m, 256), 256, 0, s, false, out_c<double2>(w), bh, m);
+    return launch_dependent(blue_mul_kernel<float2>, grid_for(m, 256), 256, 0, s, false, out_c<float2>(w), bh, m);
 }
 cudaError_t launch_blue_post(const void *w, void *out, int64_t n, const double2 *b, double scale, bool conj_out,
                              bool dbl, cudaStream_t s) {
-    ++g_launches;
+    const int cj = conj_out;
     if (dbl)
-        blue_post_kernel<double2><<<grid_for(n, 256), 256, 0, s>>>((const double2 *)w, (double2 *)out, n, b, scale,
-                                                                  conj_out);
-    else
-        blue_post_kernel<float2><<<grid_for(n, 256), 256, 0, s>>>((const float2 *)w, (float2 *)out, n, b, scale,
-                                                                 conj_out);
-    return cudaGetLastError();
+        return launch_dependent(blue_post_kernel<double2>, grid_for(n, 256), 256, 0, s, false, in_c<double2>(w),
+                                out_c<double2>(out), n, b, scale, cj);
+    return launch_dependent(blue_post_kernel<float2>, grid_for(n, 256), 256, 0, s, false, in_c<float2>(w),
+                            out_c<float2>(out), n, b, scale, cj);
 }
 cudaError_t launch_blue_transfer(void *w, void *U, bool given, int64_t n, int64_t m, const double2 *b,
                                  const PropArgs &p, bool dbl, cudaStream_t s) {
-    ++g_launches;
+    const int g = given;
     if (dbl)
-        blue_transfer_kernel<double2><<<grid_for(m, 256), 256, 0, s>>>((double2 *)w, (double2 *)U, given, n, m, b, p);
-    else blue_transfer_kernel<float2><<<grid_for(m, 256), 256, 0, s>>>((float2 *)w, (float2 *)U, given, n, m, b, p);
-    return cudaGetLastError();
+        return launch_dependent(blue_transfer_kernel<double2>, grid_for(m, 256), 256, 0, s, false, out_c<double2>(w),
+                                out_c<double2>(U), g, n, m, b, p);
+    return launch_dependent(blue_transfer_kernel<float2>, grid_for(m, 256), 256, 0, s, false, out_c<float2>(w),
+                            out_c<float2>(U), g, n, m, b, p);
 }
-cudaError_t launch_blue_table(const double2 *nat, double2 *out, int64_t m, const SpecLevels &v, int log_e,
-                              cudaStream_t s) {
-    ++g_launches;
-    blue_table_kernel<<<grid_for(m, 256), 256, 0, s>>>(nat, out, m, v, log_e);
-    return cudaGetLastError();
-}
-
 }  // namespace rsw
 
 namespace rsw {

@@ -263,6 +263,7 @@ extern "C" rsw_status rsw_fft_forward_noalloc(const void *d_in, void *d_out, int
         }
     }
     PassArgs a{};
+    a.serial = 1;  // the tables may be the preceding kernel's work
     a.n = n;
     a.log_n1 = log_n1;
     a.log_n2 = log_n2;
@@ -290,7 +291,7 @@ extern "C" rsw_status rsw_fft_forward_noalloc(const void *d_in, void *d_out, int
     a.out = spec;
     a.flags = PF_FWD;
     if ((e = launch_row_pass(a, dbl, 16, s)) != cudaSuccess) return fail_na(RSW_ERR_CUDA, cudaGetErrorString(e));
-    if ((e = launch_spec_to_natural(spec, d_out, n, SpecLevels{log_n1, 0, log_n2, 4, 4, 4}, dbl, s)) != cudaSuccess)
+    if ((e = launch_spec_to_natural(spec, d_out, n, SpecLevels{log_n1, 0, log_n2, 4, 4, 4, 4}, dbl, s)) != cudaSuccess)
         return fail_na(RSW_ERR_CUDA, cudaGetErrorString(e));
     return RSW_OK;
 }

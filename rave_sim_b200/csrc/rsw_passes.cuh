@@ -51,6 +51,18 @@ __device__ __forceinline__ void prefetch_l2_tile(const CUtensorMap *map, int x, 
                  : "memory");
 }
 
+// Programmatic dependent launch: the pass kernels are launched so that their
+// CTAs may start while the preceding kernel of the stream drains. What comes
+// before pass_wait reads only the kernel's arguments and the plan's constant
+// tables; pass_wait returns once the preceding kernel has completed (and is a
+// no-op in an ordinary launch). Every thread of every CTA calls it: a kernel
+// that completed without waiting could overtake the one before it. The next
+// kernel may start its own CTAs from then on (pass_release). The field is read
+// past L1 (__ldcg): the lines that the preceding kernel left there, on an SM
+// where both run, are not this kernel's.
+__device__ __forceinline__ void pass_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pass_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Range reduction of a phase to [-pi, pi] (Cody & Waite 1980, three-part
 // constant; 2pi = P1 + P2 + P3 with P1, P2 of 29 significant bits so that
 // k*P1 and k*P2 are exact for |k| < 2^24), then sincos of the remainder.
@@ -446,7 +458,6 @@ __global__ void __launch_bounds__(Block<Real, LOG_L2, 1, E>::NT, row_min_ctas<Re
     const int flags = a.flags;
     const int64_t rows = a.n >> LOG_L2;
     B::load_twiddles(tw, static_cast<const Tw *>(a.tw_row));
-    __syncthreads();
     const int64_t nmask = (int64_t(1) << a.tw_log) - 1;
     const double tw_scale = a.tw_scale;
     const int log_m = a.log_n1 + a.log_nb;  // spectrum index k = kbase + 2^log_m * k2
@@ -527,9 +538,16 @@ __global__ void __launch_bounds__(Block<Real, LOG_L2, 1, E>::NT, row_min_ctas<Re
                 }
             }
         }
-        if constexpr (B::NS == 1) __syncthreads();  // no barrier inside a one-stage transform
-        const Cx *__restrict__ gin = static_cast<const Cx *>(a.in) + (row << LOG_L2);
-        Cx *__restrict__ gout = static_cast<Cx *>(a.out) + (row << LOG_L2);
+        if (row == blockIdx.x) {  // what is above does not depend on the preceding kernel
+            B::twiddles_loaded();
+            pass_wait();
+            pass_release();
+            __syncthreads();
+        } else if constexpr (B::NS == 1) {
+            __syncthreads();  // no barrier inside a one-stage transform
+        }
+        const Cx *gin = static_cast<const Cx *>(a.in) + (row << LOG_L2);
+        Cx *gout = static_cast<Cx *>(a.out) + (row << LOG_L2);
         // this CTA's next row into L2 while this one is transformed, issued
         // after this row's own loads
         const auto prefetch_next = [&] {
@@ -544,7 +562,7 @@ __global__ void __launch_bounds__(Block<Real, LOG_L2, 1, E>::NT, row_min_ctas<Re
         Cx v[E];
         if (!(flags & PF_SPEC_IN)) {
 #pragma unroll
-            for (int r = 0; r < E; ++r) v[r] = (flags & PF_ONES) ? one_c<Cx>() : gin[B::first_pos(tp, r)];
+            for (int r = 0; r < E; ++r) v[r] = (flags & PF_ONES) ? one_c<Cx>() : __ldcg(gin + B::first_pos(tp, r));
             prefetch_next();
             if (TWF && (flags & PF_TWF)) {
                 __syncthreads();  // this row's factor table is complete
@@ -572,7 +590,7 @@ __global__ void __launch_bounds__(Block<Real, LOG_L2, 1, E>::NT, row_min_ctas<Re
             if (flags & PF_FWD) B::forward(sm, tp, v, tw);
         } else {
 #pragma unroll
-            for (int r = 0; r < E; ++r) v[r] = gin[B::last_pos(tp, r)];
+            for (int r = 0; r < E; ++r) v[r] = __ldcg(gin + r * B::T + tp);
             prefetch_next();
         }
 
@@ -678,7 +696,7 @@ __global__ void __launch_bounds__(Block<Real, LOG_L2, 1, E>::NT, row_min_ctas<Re
             for (int r = 0; r < E; ++r) gout[B::first_pos(tp, r)] = v[r];
         } else {
 #pragma unroll
-            for (int r = 0; r < E; ++r) gout[B::last_pos(tp, r)] = v[r];
+            for (int r = 0; r < E; ++r) gout[r * B::T + tp] = v[r];
         }
         if (!paired) __syncthreads();
     }
@@ -814,7 +832,6 @@ __device__ __forceinline__ void col_pass(const PassArgs &a) {
     const int64_t tiles = (a.n >> LOG_L1) / C;
     const int64_t nmask = (int64_t(1) << a.tw_log) - 1;
     B::load_twiddles(tw, static_cast<const Tw *>(a.tw_col));
-    __syncthreads();
     // An inverse + forward tile starts and ends with the last-stage positions
     // of each thread, so the next tile may overwrite the data buffer without
     // a barrier; every other flow ends its tile with one.
@@ -865,13 +882,20 @@ __device__ __forceinline__ void col_pass(const PassArgs &a) {
                     vec[cc * EP + (e - NXY)] = w4(a, (int64_t(B::freq_off(e - NXY)) * n2) & nmask);
             }
         }
-        if constexpr (B::NS == 1) __syncthreads();  // no barrier inside a one-stage transform
-        const Cx *__restrict__ gin = static_cast<const Cx *>(a.in) + base + col;
-        Cx *__restrict__ gout = static_cast<Cx *>(a.out) + base + col;
+        if (tile == t_first) {  // what is above does not depend on the preceding kernel
+            B::twiddles_loaded();
+            pass_wait();
+            pass_release();
+            __syncthreads();
+        } else if constexpr (B::NS == 1) {
+            __syncthreads();  // no barrier inside a one-stage transform
+        }
+        const Cx *gin = static_cast<const Cx *>(a.in) + base + col;
+        Cx *gout = static_cast<Cx *>(a.out) + base + col;
         Cx v[E];
         if (flags & PF_INV) {
 #pragma unroll
-            for (int r = 0; r < E; ++r) v[r] = gin[int64_t(B::last_pos(tp, r)) << log_n2];
+            for (int r = 0; r < E; ++r) v[r] = __ldcg(gin + (int64_t(B::last_pos(tp, r)) << log_n2));
             prefetch_next(tile);
             if (flags & PF_TWI) {
                 __syncthreads();  // this tile's factor table is complete
@@ -894,7 +918,7 @@ __device__ __forceinline__ void col_pass(const PassArgs &a) {
         } else if constexpr (!DET) {
 #pragma unroll
             for (int r = 0; r < E; ++r)
-                v[r] = (flags & PF_ONES) ? one_c<Cx>() : gin[int64_t(B::first_pos(tp, r)) << log_n2];
+                v[r] = (flags & PF_ONES) ? one_c<Cx>() : __ldcg(gin + (int64_t(B::first_pos(tp, r)) << log_n2));
             prefetch_next(tile);
         }
         // the detection variant runs the inverse only: no transmission, no forward
@@ -963,6 +987,8 @@ template <typename Real, int LOG_L2, int E>
 __global__ void chirp_table_kernel(typename LiftT<Real>::T *__restrict__ out, double g3_hi, double g3_lo) {
     using B = Block<Real, LOG_L2, 1, E>;
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    pass_wait();  // the table's last reader
+    pass_release();
     if (idx >= B::L) return;
     const int r = idx / B::T, tp = idx % B::T;
     const int half2 = 1 << (LOG_L2 - 1);
@@ -1014,6 +1040,29 @@ static const LaunchSetup *launch_setup(K kernel, int threads, size_t smem, size_
     return &table[dev];
 }
 
+// launch with programmatic dependent launch (pass_wait): the CTAs of a short
+// pass load their twiddles and build their factor tables while the pass
+// before it finishes. A split step of 2^16 complex128 samples (two launches)
+// 22.9 -> 13.4 us, 2^14 complex64 22.9 -> 10.9, 2^20 complex128 35.2 -> 29.7;
+// no change from 2^24 on.
+template <typename K, typename... Args>
+static cudaError_t launch_dependent(K kernel, int64_t grid, int threads, size_t smem, cudaStream_t s, bool serial,
+                                    const Args &...args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(unsigned(grid));
+    cfg.blockDim = dim3(unsigned(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = serial ? 0 : 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+    if (e == cudaSuccess) count_launch();
+    return e;
+}
+
 template <int L> constexpr int n_vec() { return 64 + ((L >> 6) > 0 ? (L >> 6) : 1); }
 template <int L, int E> constexpr int n_chirp() { return 64 + ((L >> 6) > 1 ? (L >> 6) : 2) + E; }
 
@@ -1029,9 +1078,7 @@ static cudaError_t row_launch(const PassArgs &a, cudaStream_t s) {
     if (st->attr != cudaSuccess) return st->attr;
     const int64_t cap = st->cap[0];
     const int64_t rows = a.n >> LG;
-    k<<<dim3(unsigned(rows < cap ? rows : cap)), dim3(B::NT), smem, s>>>(a);
-    count_launch();
-    return cudaGetLastError();
+    return launch_dependent(k, rows < cap ? rows : cap, B::NT, smem, s, a.serial != 0, a);
 }
 // PF_TWF (rows of three-level plans) takes the TWF variant, for the chirp
 // form and for the per-sample transfer function (exact kernel) alike; rows of
@@ -1099,15 +1146,11 @@ static cudaError_t col_impl(const PassArgs &a, cudaStream_t s) {
     constexpr int words = int(sizeof(typename B::Cx) / 8);
     b.in_map_ok = a.in && !(a.flags & PF_ONES) && tiles > grid &&
                   encode_col_map(&b.in_map, a.in, a.n, a.log_n2, words, C * words, B::L < 256 ? B::L : 256);
-    k<<<dim3(unsigned(grid)), dim3(B::NT), tables ? tab : plain, s>>>(b);
-    count_launch();
-    return cudaGetLastError();
+    return launch_dependent(k, grid, B::NT, tables ? tab : plain, s, a.serial != 0, b);
 }
 
 template <typename Real, int LG, int E> static cudaError_t chirp_impl(void *out, double hi, double lo, cudaStream_t s) {
-    chirp_table_kernel<Real, LG, E><<<((1 << LG) + 255) / 256, 256, 0, s>>>(
-        static_cast<typename LiftT<Real>::T *>(out), hi, lo);
-    count_launch();
-    return cudaGetLastError();
+    return launch_dependent(chirp_table_kernel<Real, LG, E>, ((1 << LG) + 255) / 256, 256, 0, s, false,
+                            static_cast<typename LiftT<Real>::T *>(out), hi, lo);
 }
 }  // namespace rsw
