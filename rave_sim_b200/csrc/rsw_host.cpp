@@ -509,22 +509,31 @@ static rsw_status plan_split(int64_t n, int dtype, int *log_n, int *l1, int *lb,
             return RSW_OK;
         }
     }
-    if (lg <= row_max) {
+    // Single rows up to 2^11 samples only: one CTA runs the whole transform,
+    // with the transfer function evaluated per sample. A propagation of 2^13
+    // complex128 samples takes 31 us on one row and 16 us as short passes, of
+    // 2^14 complex64 35 and 16 us, a forward FFT 19 and 13 us (2^14 complex64
+    // 25 and 13). At 2^11 both are equal, and the FFT is 1 us faster on one row.
+    if (lg <= 11) {
         *l1 = 0;
         *lr = lg;
         return RSW_OK;
     }
+    const bool c128 = dtype == RSW_C128;
     const int col2 = dtype == RSW_C128 ? COL_TUNE_MAX_C128 : col_max;  // two-level column limit
     if (lg > row_max + col2) {
         if (lg > row_max + 2 * col_max)
             return fail(RSW_ERR_UNSUPPORTED, "N = 2^%d exceeds the three-level limit 2^%d for this dtype", lg,
                         row_max + 2 * col_max);
-        // long outer columns (the pass with the transmission and the factor
-        // tables, which amortise over the column length); the middle level
-        // runs plain FFTs of what is left, at least 2^4
+        // outer columns of 2^8 and the rest in the middle while that stays
+        // short (split step at 2^26 complex128: 2.53 ms against 2.59 for
+        // columns of 2^9; 2^27 complex128 5.03 against 5.61 for 2^10, complex64
+        // 2.98 against 3.06 for 2^9); beyond, long outer columns (the pass
+        // with the transmission and the factor tables, which amortise over
+        // the column length) and the rest in the middle, at least 2^4
         const int rest = lg - row_max;
         *lr = row_max;
-        *l1 = std::min(std::min(col_max, 11), rest - 4);
+        *l1 = rest <= 14 ? 8 : std::min(std::min(col_max, 11), rest - 4);
         *lb = rest - *l1;
         if (*lb > col_max) {
             *lb = col_max;
@@ -532,18 +541,18 @@ static rsw_status plan_split(int64_t n, int dtype, int *log_n, int *l1, int *lb,
         }
         return RSW_OK;
     }
-    // prefer columns of at most 2^11 (the 2^12 c64 column kernel runs 1024
-    // threads at 64 registers and spills); rows take the rest
-    int a = std::min(std::min(col_max, 11), lg / 2);
+    // Two levels. Short fields: rows of 2^7 or 2^8, enough of them for every
+    // SM. complex128 from 2^20: rows of 2^12, of which two run on an SM (split
+    // step at 2^20 31.5 us against 36.8 for rows of 2^10, 2^21 58 against 67,
+    // 2^22 117 against 121 for 2^11, 2^24 461 against 487 for 2^13). complex64
+    // keeps columns of at most 2^11 (those of 2^12 spill at 64 registers),
+    // and the longer rows at 2^18 (12.1 against 13.4 us) and 2^20 (22 against
+    // 26). In between even halves.
+    int a = lg <= 14 ? lg - 8 + (lg < 14) : lg / 2;
+    if (c128 && lg >= 20) a = std::min(lg - 12, COL_TUNE_MAX_C128);
+    if (!c128 && (lg == 18 || lg == 20)) --a;
+    if (!c128) a = std::min(a, 11);
     int b = lg - a;
-    if (b > row_max) {
-        a = lg - row_max;
-        b = row_max;
-    }
-    if (b < 7) {  // rows of two-level plans hold at least 2^7 samples
-        b = 7;
-        a = lg - b;
-    }
     if (b > row_max) {
         a = lg - row_max;
         b = row_max;
@@ -554,14 +563,14 @@ static rsw_status plan_split(int64_t n, int dtype, int *log_n, int *l1, int *lb,
 }
 
 // Kernel variant per block size: elements per thread. complex128 columns of
-// 2^8 .. 2^11 take 8 per thread (radix-8 stages, 512- or 1024-thread CTAs:
-// two to four times the warps per SM of the 16-per-thread kernels, which
-// hold up to 252 registers at 256 threads; measured 9-20 % faster), as do
-// complex64 columns of 2^9 (16 per CTA, 6 %) and of 2^10 in two-level plans
-// (at most 2^21 samples: too few tiles of 16 columns for 148 SMs). Other
-// complex64 columns of 2^10 and 2^11 keep 16 per thread, which leaves room
-// for 16 or 8 columns per CTA (128- or 64-byte row segments; 8 per thread
-// with 4 columns measured 26-40 % slower). Everything else takes 16.
+// 2^8 .. 2^12 of two-level plans take 8 per thread (radix-8 stages, 512- or
+// 1024-thread CTAs: two to four times the warps per SM of the 16-per-thread
+// kernels; measured 9-20 % faster), as do complex64 columns of 2^9 (16 per
+// CTA, 6 %). Other complex64 columns keep 16 per thread, which leaves room
+// for 16 or 8 columns per CTA (128- or 64-byte row segments; 2^21 samples in
+// columns of 2^10: 40 us a split step against 49 with 8 per thread and 4
+// columns), and so do the outer columns of three-level plans (2^26 complex128
+// 2.53 against 2.59 ms). Everything else takes 16.
 // RSW_ROW_E / RSW_COL_E (8, 16 or 32) override the choice (tuning sweeps).
 static int env_int(const char *name, int dflt) {
     const char *v = std::getenv(name);
@@ -584,7 +593,7 @@ static rsw_status choose_tuning(rsw_plan_s *p, const rsw_tuning *t) {
     p->row_e = pick(p->log_nr, 16);
     const bool c128 = p->dtype == RSW_C128;
     const int l1 = p->log_n1;
-    p->col_e = (c128 && l1 >= 8 && l1 <= 12) || (!c128 && (l1 == 9 || (l1 == 10 && p->log_nb == 0))) ? 8 : pick(l1, 16);
+    p->col_e = (c128 && l1 >= 8 && l1 <= 12 && p->log_nb == 0) || (!c128 && l1 == 9) ? 8 : pick(l1, 16);
     p->mid_e = pick(p->log_nb, 16);
     if (t) {
         const bool multi = p->log_n1 > 0;
