@@ -2,7 +2,7 @@
 //
 // A "block" transforms C independent sequences of length L = 2^LOG_L held by
 // one CTA. Each thread owns E = 8, 16 or 32 elements in registers; stages are
-// radix-8 (E = 8) or radix-16, the last one takes the remaining radix
+// radix E, the last one takes the remaining radix
 // (rsw_stages.h).
 // Forward stages are decimation in frequency: natural order in,
 // digit-reversed order out. Inverse stages are the exact mirror (decimation
@@ -211,6 +211,52 @@ template <int DIR> __device__ __forceinline__ float2 tw16(float2 x, int e) {
     }
 }
 
+// x * W32^e with W32 = exp(DIR * 2 pi i / 32), e in [0, 16), e known after
+// unrolling: the rotations above at even e, otherwise as they are (FP64: a
+// product; FP32: shears of at most 3 pi / 16 after exact quarter turns).
+template <int DIR> __device__ __forceinline__ double2 tw32_odd(double2 x, int e) {
+    const double c1 = 0.98078528040323044913, s1 = 0.19509032201612826785;  // pi / 16
+    const double c3 = 0.83146961230254523708, s3 = 0.55557023301960222474;  // 3 pi / 16
+    const double d = double(DIR);
+    switch (e) {
+    case 1: return cmul(x, mk(c1, d * s1));
+    case 3: return cmul(x, mk(c3, d * s3));
+    case 5: return cmul(x, mk(s3, d * c3));
+    case 7: return cmul(x, mk(s1, d * c1));
+    case 9: return cmul(x, mk(-s1, d * c1));
+    case 11: return cmul(x, mk(-s3, d * c3));
+    case 13: return cmul(x, mk(-c3, d * s3));
+    default: return cmul(x, mk(-c1, d * s1));
+    }
+}
+template <int DIR, int EE> __device__ __forceinline__ float2 tw32_lift(float2 x) {
+    constexpr int q = EE <= 4 ? 0 : EE <= 12 ? -1 : -2;
+    constexpr int t = -EE - 8 * q;  // -3, -1, 1 or 3
+    constexpr float A1 = 0.098491403357164253077f;  // tan(pi/32)
+    constexpr float B1 = 0.19509032201612826785f;   // sin(pi/16)
+    constexpr float A3 = 0.30334668360734239168f;   // tan(3 pi/32)
+    constexpr float B3 = 0.55557023301960222474f;   // sin(3 pi/16)
+    constexpr float a = t == -3 ? A3 : t == -1 ? A1 : t == 1 ? -A1 : -A3;
+    constexpr float b = t == -3 ? -B3 : t == -1 ? -B1 : t == 1 ? B1 : B3;
+    if constexpr (DIR < 0) return quarter<q>(lift(x, a, b));
+    else return lift(quarter<-q>(x), -a, -b);
+}
+template <int DIR> __device__ __forceinline__ float2 tw32_odd(float2 x, int e) {
+    switch (e) {
+    case 1: return tw32_lift<DIR, 1>(x);
+    case 3: return tw32_lift<DIR, 3>(x);
+    case 5: return tw32_lift<DIR, 5>(x);
+    case 7: return tw32_lift<DIR, 7>(x);
+    case 9: return tw32_lift<DIR, 9>(x);
+    case 11: return tw32_lift<DIR, 11>(x);
+    case 13: return tw32_lift<DIR, 13>(x);
+    default: return tw32_lift<DIR, 15>(x);
+    }
+}
+template <int DIR, typename C> __device__ __forceinline__ C tw32(C x, int e) {
+    return (e & 1) ? tw32_odd<DIR>(x, e) : tw16<DIR>(x, e >> 1);
+}
+
 // Radix-2 decimation-in-frequency network: natural order in, bit-reversed out.
 template <int R, int DIR, typename C> __device__ __forceinline__ void net_dif(C *v) {
 #pragma unroll
@@ -221,7 +267,7 @@ template <int R, int DIR, typename C> __device__ __forceinline__ void net_dif(C 
             for (int k = 0; k < span; ++k) {
                 C a = v[start + k], b = v[start + k + span];
                 v[start + k] = cadd(a, b);
-                v[start + k + span] = tw16<DIR>(csub(a, b), k * (8 / span));
+                v[start + k + span] = tw32<DIR>(csub(a, b), k * (16 / span));
             }
         }
     }
@@ -234,7 +280,7 @@ template <int R, int DIR, typename C> __device__ __forceinline__ void net_dit(C 
         for (int start = 0; start < R; start += 2 * span) {
 #pragma unroll
             for (int k = 0; k < span; ++k) {
-                C a = v[start + k], b = tw16<DIR>(v[start + k + span], k * (8 / span));
+                C a = v[start + k], b = tw32<DIR>(v[start + k + span], k * (16 / span));
                 v[start + k] = cadd(a, b);
                 v[start + k + span] = csub(a, b);
             }
@@ -270,8 +316,8 @@ template <int LOG_L, int E_ = 16, int MAX_LS = 7> struct Radix {
 };
 
 template <typename Real, int LOG_L, int C, int E_ = 16>
-struct Block : Radix<LOG_L, E_, direct_max_ls(2 * sizeof(Real), LOG_L)> {
-    using Rx = Radix<LOG_L, E_, direct_max_ls(2 * sizeof(Real), LOG_L)>;
+struct Block : Radix<LOG_L, E_, direct_max_ls(2 * sizeof(Real), LOG_L, digit_bits(E_))> {
+    using Rx = Radix<LOG_L, E_, direct_max_ls(2 * sizeof(Real), LOG_L, digit_bits(E_))>;
     using Cx = typename CxT<Real>::T;
     using Tw = typename TwT<Real>::T;  // twiddle table entry (16 bytes)
     static constexpr bool LIFT = sizeof(Real) == 4;  // complex64: rotations by lifting

@@ -11,9 +11,9 @@ namespace rsw {
 // 8 or 16 samples per thread (C8 / C16 columns per CTA), 32 on request
 #define RSW_COL_CASE_E(R, L, C8, C16)                                                       \
     case L: return e == 8 ? col_impl<R, L, C8, 8, DET, BT>(a, s)                           \
-                          : e == 32 ? col_impl<R, L, 4, 32, DET, BT>(a, s) : col_impl<R, L, C16, 16, DET, BT>(a, s);
+                          : e == 32 ? col_impl<R, L, col_c32<R>(L), 32, DET, BT>(a, s) : col_impl<R, L, C16, 16, DET, BT>(a, s);
 #define RSW_COL_CASE(R, L) \
-    case L: return e == 32 ? col_impl<R, L, 4, 32, DET, BT>(a, s) : col_impl<R, L, col_c(L), 16, DET, BT>(a, s);
+    case L: return e == 32 ? col_impl<R, L, col_c32<R>(L), 32, DET, BT>(a, s) : col_impl<R, L, col_c(L), 16, DET, BT>(a, s);
 
 // Columns per CTA: col_c(L) (16-byte samples: 64- to 512-byte row
 // segments); complex64 doubles them where the threads allow (col_c64).

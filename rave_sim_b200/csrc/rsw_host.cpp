@@ -325,6 +325,7 @@ struct rsw_plan_s {
     int log_nb = 0, log_nr = 0;  // N2 = Nb * Nr: middle level (0: two-level) and row-kernel length
     int device = 0;
     int row_e = 16, col_e = 16, mid_e = 16;  // elements per thread of the row / column / middle kernels
+    bool row_tuned = false;                  // row_e was asked for (a tuning, RSW_ROW_E)
     int prop_mode = RSW_PROP_FRESNEL;        // transfer function of propagate and of simulations
     DevBuf tw_row, tw_col, tw_mid, tw4_lo, tw4_hi, tw4b_lo, tw4b_hi;
     int tw4_shift = 0, tw4b_shift = 0;
@@ -404,7 +405,7 @@ template <typename T> static std::vector<T> block_twiddles(int log_l, int rb) {
     std::vector<T> v;
     constexpr bool lift = sizeof(T) == 4;
     if (log_l >= 4) {
-        const int max_ls = direct_max_ls(int(2 * sizeof(T)), log_l);
+        const int max_ls = direct_max_ls(int(2 * sizeof(T)), log_l, rb);
         for (int s = 0; s < stage_count(log_l, rb) - 1; ++s) {
             for (int64_t k = 0; k < stage_tw_entries(log_l, s, max_ls, rb); ++k) {
                 int64_t m, mod;
@@ -590,7 +591,10 @@ static bool col_e_ok(int log_l, int e, bool c128) {
 
 static rsw_status choose_tuning(rsw_plan_s *p, const rsw_tuning *t) {
     auto pick = [](int log_l, int dflt) { return log_l >= 9 ? dflt : 16; };
-    p->row_e = pick(p->log_nr, 16);
+    // complex64 rows of 2^14 in radix 32: three stages and two exchanges per
+    // direction in place of four and three (split step at 2^26 1.32 -> 1.27
+    // ms, 2^25 548 -> 536 us; at 2^13 the 32 warps of radix 16 are as fast)
+    p->row_e = p->dtype == RSW_C64 && p->log_n1 > 0 && p->log_nr == 14 ? 32 : pick(p->log_nr, 16);
     const bool c128 = p->dtype == RSW_C128;
     const int l1 = p->log_n1;
     p->col_e = (c128 && l1 >= 8 && l1 <= 12 && p->log_nb == 0) || (!c128 && l1 == 9) ? 8 : pick(l1, 16);
@@ -607,12 +611,14 @@ static rsw_status choose_tuning(rsw_plan_s *p, const rsw_tuning *t) {
             return fail(RSW_ERR_INVALID, "tuning: no middle kernel of 2^%d with %d samples per thread", p->log_nb,
                         t->mid_e);
         if (t->row_e) p->row_e = t->row_e;
+        p->row_tuned = t->row_e != 0;
         if (t->col_e) p->col_e = t->col_e;
         if (t->mid_e) p->mid_e = t->mid_e;
         return RSW_OK;
     }
     const int re = env_int("RSW_ROW_E", 0), ce = env_int("RSW_COL_E", 0);
     if ((re == 16 || re == 32) && p->log_nr >= 9) p->row_e = re;
+    p->row_tuned = re == 8 || re == 16 || re == 32;
     if (ce == 16 || (ce == 32 && p->log_n1 >= 9)) p->col_e = ce;
     // 8 samples per thread: multi-level rows of 2^11..2^13, columns of 2^8..2^11
     if (re == 8 && p->log_n1 > 0 && p->log_nr >= 11 && p->log_nr <= 13) p->row_e = 8;
@@ -911,7 +917,9 @@ static rsw_status create_blue_plan(rsw_plan *out, int64_t n, int dtype) {
     rsw_plan inner = nullptr;
     rsw_tuning reg{};
     const bool use = !env_overrides() && registered_tuning(m, dtype, &reg);
-    CHECK(create_plan(&inner, m, dtype, use ? &reg : nullptr));
+    rsw_tuning rows16{};  // the table product's row kernels, unless a tuning asks for others
+    rows16.row_e = 16;
+    CHECK(create_plan(&inner, m, dtype, use ? &reg : env_overrides() ? nullptr : &rows16));
     p->inner.reset(inner);
     // chirp b[k] = exp(i pi k^2 / n), k^2 reduced mod 2n exactly
     const long double pi = 3.14159265358979323846264338327950288L;
@@ -1191,9 +1199,18 @@ rsw_status rsw_plan_info(rsw_plan p, int64_t *n, int *dtype, int *log_rows, int 
 rsw_status rsw_plan_set_propagator(rsw_plan p, int mode) {
     if (!p) return fail(RSW_ERR_INVALID, "plan is NULL");
     if (mode != RSW_PROP_FRESNEL && mode != RSW_PROP_EXACT) return fail(RSW_ERR_INVALID, "unknown propagator %d", mode);
-    // the exact kernel runs the per-sample row kernels (16 samples per thread)
-    if (mode == RSW_PROP_EXACT && p->log_n1 > 0 && p->row_e != 16)
-        return fail(RSW_ERR_UNSUPPORTED, "the exact propagator needs rows of 16 samples per thread");
+    // the exact kernel runs the per-sample row kernels (16 samples per
+    // thread): a plan whose rows took another count by default changes over
+    if (mode == RSW_PROP_EXACT && p->log_n1 > 0 && p->row_e != 16) {
+        if (p->row_tuned)
+            return fail(RSW_ERR_UNSUPPORTED, "the exact propagator needs rows of 16 samples per thread");
+        DevBuf tw;
+        CHECK(p->dbl() ? tw.upload(block_twiddles<double>(p->log_nr, digit_bits(16)))
+                       : tw.upload(block_twiddles<float>(p->log_nr, digit_bits(16))));
+        CU(cudaDeviceSynchronize());  // the old table's readers
+        p->tw_row = std::move(tw);
+        p->row_e = 16;
+    }
     p->prop_mode = mode;
     return RSW_OK;
 }

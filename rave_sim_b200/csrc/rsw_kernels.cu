@@ -84,10 +84,10 @@ template <int RB> __device__ __forceinline__ int digitpos_32(int f, int log_l) {
     return p;
 }
 __device__ __forceinline__ int digitrev_i(int p, int log_l, int rb) {
-    return rb == 3 ? digitrev_32<3>(p, log_l) : digitrev_32<4>(p, log_l);
+    return rb == 3 ? digitrev_32<3>(p, log_l) : rb == 5 ? digitrev_32<5>(p, log_l) : digitrev_32<4>(p, log_l);
 }
 __device__ __forceinline__ int digitpos_i(int f, int log_l, int rb) {
-    return rb == 3 ? digitpos_32<3>(f, log_l) : digitpos_32<4>(f, log_l);
+    return rb == 3 ? digitpos_32<3>(f, log_l) : rb == 5 ? digitpos_32<5>(f, log_l) : digitpos_32<4>(f, log_l);
 }
 // a thread's register number <-> offset among its E block positions
 // (Block::last_off, its own inverse): the low lrl bits reversed, lrl the log2

@@ -64,7 +64,7 @@ constexpr size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 // thread, radix-16 stages; 16-byte entries for complex128, 8 for complex64)
 constexpr size_t block_tw_bytes(int log_l, bool dbl) {
     const int eb = dbl ? 16 : 8;
-    const int max_ls = direct_max_ls(eb, log_l);
+    const int max_ls = direct_max_ls(eb, log_l, 4);
     int64_t n = 0;
     for (int s = 0; s < stage_count(log_l) - 1; ++s) n += stage_tw_entries(log_l, s, max_ls);
     return size_t(n > 0 ? n : 1) * size_t(eb);
@@ -115,7 +115,7 @@ namespace {
 template <typename T>
 __device__ void block_tables(T *out, int log_l, int idx, int stride) {
     int off = 0;
-    const int max_ls = direct_max_ls(int(2 * sizeof(T)), log_l);
+    const int max_ls = direct_max_ls(int(2 * sizeof(T)), log_l, 4);
     for (int s = 0; s < stage_count(log_l) - 1; ++s) {
         const int count = stage_tw_entries(log_l, s, max_ls);
         for (int k = idx; k < count; k += stride) {

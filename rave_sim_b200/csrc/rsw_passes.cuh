@@ -386,9 +386,9 @@ __device__ __forceinline__ double2 w4(const PassArgs &a, int64_t m) {
     return cmul(__ldg(lo + (m & mask)), __ldg(hi + (m >> a.tw4_shift)));
 }
 
-// digitrev_rt with the digit width as a compile-time constant (3 or 4)
+// digitrev_rt with the digit width as a compile-time constant (3, 4 or 5)
 __device__ __forceinline__ int64_t digitrev_w(int64_t p, int log_l, int rb) {
-    return rb == 3 ? digitrev_rt(p, log_l, 3) : digitrev_rt(p, log_l, 4);
+    return rb == 3 ? digitrev_rt(p, log_l, 3) : rb == 5 ? digitrev_rt(p, log_l, 5) : digitrev_rt(p, log_l, 4);
 }
 
 // ceil(x / 2^log_n1) clamped to [0, l]: the first row frequency k2 with
@@ -429,9 +429,11 @@ template <int T> struct ColTab {
 // 14.0; 24 warps at 80 registers: 24.3 and 14.0. Rows of 2^13 and more fill
 // the SM at these counts anyway. Shorter rows stay uncapped: the caps made
 // them spill in the factor tables' sincospi (complex128 2^10 2 %, 2^8 7 % and
-// 2^11 forward rows 10 % slower). So do single rows (no chirp form).
+// 2^11 forward rows 10 % slower). So do single rows (no chirp form). Radix-32
+// rows of complex64 run 16 warps at 128 registers.
 template <typename Real, int LOG_L2, int E, bool CHIRP> constexpr int row_min_ctas() {
-    if (E == 32 || LOG_L2 < (sizeof(Real) == 8 && E == 16 ? 12 : 11)) return 1;
+    if (E == 32) return sizeof(Real) == 4 && LOG_L2 >= 10 && LOG_L2 < 14 ? 512 / ((1 << LOG_L2) / 32) : 1;
+    if (LOG_L2 < (sizeof(Real) == 8 && E == 16 ? 12 : 11)) return 1;
     if (!CHIRP && !(sizeof(Real) == 4 && LOG_L2 == 13)) return 1;
     constexpr int want = (sizeof(Real) == 8 && E == 16 ? 512 : 1024) / ((1 << LOG_L2) / E);
     return want < 1 ? 1 : want;
@@ -972,7 +974,7 @@ __global__ void __launch_bounds__(Block<Real, LOG_L1, C, E>::NT) col_pass_kernel
     col_pass<Real, LOG_L1, C, E, DET, BATCH>(a);
 }
 template <typename Real, int LOG_L1, int C, int E> constexpr bool col_two_ctas() {
-    return sizeof(Real) == 8 && Block<Real, LOG_L1, C, E>::NT == 256;
+    return (sizeof(Real) == 8 || E == 32) && Block<Real, LOG_L1, C, E>::NT == 256;
 }
 template <typename Real, int LOG_L1, int C, int E, bool DET = false, bool BATCH = false>
 __global__ void __launch_bounds__(Block<Real, LOG_L1, C, E>::NT, 2)
@@ -1107,6 +1109,13 @@ constexpr int col_c(int log_l) {
 // segments, measured 26 % and 13 % faster than 32-byte ones at 2^28 and 2^24)
 constexpr int col_c64(int log_l) { return log_l == 10 ? 16 : log_l == 11 ? 8 : col_c(log_l); }
 
+// columns per CTA of the radix-32 kernels (32 samples per thread): complex64
+// 2^9 and 2^10 in 64 KB tiles of 256 threads, two on an SM
+template <typename Real> constexpr int col_c32(int log_l) {
+    if (sizeof(Real) == 8) return 4;
+    return log_l == 9 ? 16 : log_l <= 11 ? 8 : 4;
+}
+
 // The input's TMA map for the column kernel's next-tile prefetch: rows of
 // 2^log_n2 samples of words_per_sample 8-byte words, boxes of box_w words by
 // box_h rows. False (no prefetch) when the input is not 16-byte aligned or
@@ -1118,7 +1127,7 @@ template <typename Real, int LG, int C, int E, bool DET = false, bool BT = false
 static cudaError_t col_impl(const PassArgs &a, cudaStream_t s) {
     using B = Block<Real, LG, C, E>;
     auto k = [] {
-        if constexpr (col_two_ctas<Real, LG, C, E>() && !BT) return col_pass_kernel_2cta<Real, LG, C, E, DET, BT>;
+        if constexpr (col_two_ctas<Real, LG, C, E>() && (!BT || sizeof(Real) == 4)) return col_pass_kernel_2cta<Real, LG, C, E, DET, BT>;
         else return col_pass_kernel<Real, LG, C, E, DET, BT>;
     }();
     // the per-column factor tables only when the pass applies a four-step twiddle

@@ -3,8 +3,7 @@
 // entry point, so that all three agree on one layout.
 //
 // A block of length L = 2^log_l is transformed in NS = ceil(log_l / rb)
-// stages of digit width rb (radix 2^rb: 16 for kernels with 16 or 32 samples
-// per thread, 8 for 8 samples per thread), the remainder radix last. Stage s
+// stages of digit width rb (radix 2^rb: the samples per thread, 8, 16 or 32), the remainder radix last. Stage s
 // has radix R_s = 2^lr(s) and stride S_s = 2^ls(s), with
 // ls(s) = log_l - (lr(0) + ... + lr(s)); the last stage has stride 1.
 // Forward stages are decimation in frequency (large strides first), so the
@@ -31,12 +30,13 @@ namespace rsw {
 
 // Complex64 blocks of 2^13 (the two-level rows) use the factored form above
 // 2^7 too: their smaller tables let two 512-thread CTAs share an SM.
-RSW_HD constexpr int direct_max_ls(int elem_bytes, int log_l = 0) {
-    return elem_bytes <= 8 && log_l != 13 ? 9 : 7;
+// So do the radix-32 kernels, whose tables are twice as long.
+RSW_HD constexpr int direct_max_ls(int elem_bytes, int log_l, int rb) {
+    return elem_bytes <= 8 && log_l != 13 && rb != 5 ? 9 : 7;
 }
 
 // digit width of the kernels with e samples per thread
-RSW_HD constexpr int digit_bits(int e) { return e == 8 ? 3 : 4; }
+RSW_HD constexpr int digit_bits(int e) { return e == 8 ? 3 : e == 32 ? 5 : 4; }
 
 RSW_HD constexpr int stage_count(int log_l, int rb = 4) { return log_l <= 0 ? 0 : (log_l + rb - 1) / rb; }
 RSW_HD constexpr int stage_lr(int log_l, int s, int rb = 4) {
