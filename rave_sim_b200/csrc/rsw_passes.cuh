@@ -442,24 +442,69 @@ template <typename Real, int LOG_L2, int E, bool CHIRP> constexpr int row_min_ct
 // transform (a separate kernel, so that the two-level one carries no code for it).
 // BATCH: the batched variant (per-instance transfer functions, a.bpr; chirp
 // form only), also a separate kernel so that the others carry no code for it.
+// Entries of the row kernel's per-row factor tables. Rows of more than 64
+// threads keep NV = 64 + L/64 four-step factors and NCH = 64 + NQ + E chirp
+// factors and multiply two of each. For shorter rows those tables are longer
+// than the row has threads, and filling them took most of the kernel: there
+// (SHORT) each thread takes its own part of both factors directly, one
+// sincospi and one table product, and only the E register parts are shared.
+template <int LOG_L2, int E> struct RowTab {
+    static constexpr int L = 1 << LOG_L2;
+    static constexpr bool SHORT = L / E <= 64;
+    static constexpr int NQ = (L >> 6) > 1 ? (L >> 6) : 2;  // k2s >> 6 spans [-NQ/2, NQ/2)
+    static constexpr int NV = SHORT ? E : 64 + ((L >> 6) > 0 ? (L >> 6) : 1);
+    static constexpr int RO = SHORT ? 0 : 64 + NQ;  // first register part of the chirp factors
+    static constexpr int NCH = RO + E;
+};
+// Threads of the row kernel. Single rows of at most 2^11 samples evaluate the
+// transfer function per sample in FP64: 256 threads fill a table of it in
+// shared memory before the kernel waits for the one before it, then all but
+// the row's own leave (launched so only where the table is used).
+template <int LOG_L2, int NT, bool CHIRP> constexpr int row_threads() { return !CHIRP && LOG_L2 <= 11 ? 256 : NT; }
+
 template <typename Real, int LOG_L2, int E, bool CHIRP, bool TWF = false, bool BATCH = false>
-__global__ void __launch_bounds__(Block<Real, LOG_L2, 1, E>::NT, row_min_ctas<Real, LOG_L2, E, CHIRP>()) row_pass_kernel(PassArgs a) {
+__global__ void __launch_bounds__(row_threads<LOG_L2, Block<Real, LOG_L2, 1, E>::NT, CHIRP>(),
+                                  row_min_ctas<Real, LOG_L2, E, CHIRP>()) row_pass_kernel(PassArgs a) {
     using B = Block<Real, LOG_L2, 1, E>;
     using Cx = typename B::Cx;
+    using RT = RowTab<LOG_L2, E>;
     constexpr int L = B::L;
-    constexpr int NV = 64 + (L >> 6 > 0 ? L >> 6 : 1);
+    constexpr int NV = RT::NV, NQ = RT::NQ, NCH = RT::NCH, RO = RT::RO;
+    constexpr bool SHORT = RT::SHORT;
     using Tw = typename B::Tw;
     using Lf = typename LiftT<Real>::T;
     extern __shared__ __align__(16) unsigned char smraw[];
     Cx *sm = reinterpret_cast<Cx *>(smraw);
     Tw *tw = reinterpret_cast<Tw *>(smraw + B::DATA);
     Lf *const tabs = reinterpret_cast<Lf *>(smraw + (B::SMEM + 15) / 16 * 16);
-    constexpr int NQ = (L >> 6) > 1 ? (L >> 6) : 2;  // k2s >> 6 spans [-NQ/2, NQ/2)
-    constexpr int NCH = 64 + NQ + E;  // chirp factors per row: P, Q and the per-register R
     const int tp = threadIdx.x;
     const int flags = a.flags;
     const int64_t rows = a.n >> LOG_L2;
-    B::load_twiddles(tw, static_cast<const Tw *>(a.tw_row));
+    constexpr int HT = row_threads<LOG_L2, B::NT, CHIRP>();
+    if (HT == B::NT || tp < B::NT) B::load_twiddles(tw, static_cast<const Tw *>(a.tw_row));
+    // the transfer function of a single row, register r of thread t at r * T + t;
+    // (0, 0) marks a zeroed component (the others have modulus 1)
+    double2 *const hs = reinterpret_cast<double2 *>(tabs);
+    bool h_table = false;
+    if constexpr (HT > B::NT) {
+        h_table = blockDim.x > B::NT;
+        if (h_table) {
+            for (int k = tp; k < L; k += HT) {
+                double2 H = make_double2(0.0, 0.0);
+                double s, c, ph;
+                if (!(a.pr.has_cut && k >= a.pr.cut_lo && k < a.pr.cut_hi) &&
+                    prop_phase_any(a.pr, k >= L / 2 ? int64_t(k) - L : int64_t(k), &ph)) {
+                    sincos_phase(ph, &s, &c);
+                    H = make_double2(a.pr.A.x * c - a.pr.A.y * s, a.pr.A.x * s + a.pr.A.y * c);
+                }
+                const int p = int(digitpos_rt(k, LOG_L2, B::RB)), o = p % E;
+                const int r = o / B::RL * B::RL + brev_bits(o % B::RL, ilog2(B::RL));
+                hs[r * B::T + p / E] = H;
+            }
+            __syncthreads();
+            if (tp >= B::NT) return;
+        }
+    }
     const int64_t nmask = (int64_t(1) << a.tw_log) - 1;
     const double tw_scale = a.tw_scale;
     const int log_m = a.log_n1 + a.log_nb;  // spectrum index k = kbase + 2^log_m * k2
@@ -477,9 +522,12 @@ __global__ void __launch_bounds__(Block<Real, LOG_L2, 1, E>::NT, row_min_ctas<Re
         // 16-byte entries; complex64 keeps the lifting form {a, b, s, 0} of
         // each factor, except P and Q, kept in FP64 (their product is taken once
         // per row and thread before it is turned into a rotation)
-        Lf *vec = tabs + parity * (NV + NCH);  // four-step factors: [0,64) low, [64, NV) high
-        // chirp factors: [0,64) P[a], [64, 64+NQ) Q[b + NQ/2], [64+NQ, NCH) R[r]
+        // four-step factors: [0,64) low, [64, NV) high (SHORT: per register)
+        Lf *vec = tabs + parity * (NV + NCH);
+        // chirp factors: [0,64) P[a], [64, 64+NQ) Q[b + NQ/2], [RO, NCH) R[r]
         Lf *chp = vec + NV;
+        [[maybe_unused]] double2 thread_chirp = make_double2(1.0, 0.0);  // SHORT: this thread's P Q
+        [[maybe_unused]] Lf thread_tw{};                                 // SHORT: its four-step factor
         // row -> (p1, pb): spectrum index base kbase = k1 + N1 kb; the
         // conjugate four-step twiddle of the innermost split uses tw_k
         // (rows beyond one transform belong to the next one of a batch)
@@ -506,20 +554,21 @@ __global__ void __launch_bounds__(Block<Real, LOG_L2, 1, E>::NT, row_min_ctas<Re
             const double m = double(int64_t(1) << log_m);
             const double gk = frac_dd(g_hi, g_lo, double(kbase * kbase));
             const double g1h = 2.0 * m * g_hi, g1l = 2.0 * m * g_lo;
+            if constexpr (SHORT) thread_chirp = cmul(A, cis_turns(gk + frac_dd(g1h, g1l, double(kbase * fbase))));
             for (int idx = tp; idx < NCH; idx += B::NT) {
                 double2 w;
-                if (idx < 64) {
+                if (!SHORT && idx < 64) {
                     w = cmul(A, cis_turns(gk + frac_dd(g1h, g1l, double(kbase * idx))));
-                } else if (idx < 64 + NQ) {
+                } else if (!SHORT && idx < 64 + NQ) {
                     const int64_t b = int64_t(idx - 64) - NQ / 2;
                     w = cis_turns(frac_dd(g1h, g1l, double(kbase * 64 * b)));
                 } else {
-                    const int fo = B::freq_off(idx - 64 - NQ);
+                    const int fo = B::freq_off(idx - RO);
                     const int64_t sr = (fo & (L >> 1)) ? int64_t(fo) - L : int64_t(fo);
                     w = cis_turns(frac_dd(g1h, g1l, double(kbase * sr)));
                 }
                 if constexpr (B::LIFT) {
-                    if (idx < 64 + NQ) reinterpret_cast<double2 *>(chp)[idx] = w;
+                    if (idx < RO) reinterpret_cast<double2 *>(chp)[idx] = w;
                     else chp[idx] = lift_of(w);
                 } else {
                     chp[idx] = w;
@@ -527,20 +576,33 @@ __global__ void __launch_bounds__(Block<Real, LOG_L2, 1, E>::NT, row_min_ctas<Re
             }
         }
         if (flags & (PF_TW | PF_TWF)) {
-            // conj(W_M^{n2 tw_k}) * tw_scale = conj(A[n2 & 63]) * conj(B[n2 >> 6]) * tw_scale
-            for (int idx = tp; idx < NV; idx += B::NT) {
-                const int64_t m = ((idx < 64 ? int64_t(idx) : int64_t(idx - 64) << 6) * tw_k) & nmask;
-                double2 w = w4(a, m);
+            // conj(W_M^{n2 tw_k}) * tw_scale = conj(A[n2 & 63]) * conj(B[n2 >> 6]) * tw_scale;
+            // SHORT: n2 = tp + first_pos(0, r), the thread's part times the register's
+            const auto factor = [&](int64_t n2, double scale) {
+                double2 w = w4(a, (n2 * tw_k) & nmask);
                 w = make_double2(w.x, -w.y);
-                if constexpr (B::LIFT) {
-                    vec[idx] = lift_of(w, idx >= 64 ? tw_scale : 1.0);
-                } else {
-                    if (idx >= 64) w = make_double2(w.x * tw_scale, w.y * tw_scale);
-                    vec[idx] = w;
-                }
+                if constexpr (B::LIFT) return lift_of(w, scale);
+                else return make_double2(w.x * scale, w.y * scale);
+            };
+            if constexpr (SHORT) thread_tw = factor(tp, 1.0);
+            for (int idx = tp; idx < NV; idx += B::NT) {
+                if constexpr (SHORT) vec[idx] = factor(B::first_pos(0, idx), tw_scale);
+                else vec[idx] = factor(idx < 64 ? idx : int64_t(idx - 64) << 6, idx < 64 ? 1.0 : tw_scale);
             }
         }
+        // the two parts of the four-step factor of register r
+        const auto tw_thread = [&](int r) { return SHORT ? thread_tw : vec[B::first_pos(tp, r) & 63]; };
+        const auto tw_register = [&](int r) { return SHORT ? vec[r] : vec[64 + (B::first_pos(tp, r) >> 6)]; };
         if (row == blockIdx.x) {  // what is above does not depend on the preceding kernel
+            if constexpr (SHORT && CHIRP) {
+                // the row's chirp table into L1 (two launches before this one
+                // wrote it: a column pass, which waited for it, lies between)
+                if (a.pr.has_h) {
+                    const char *h3 = static_cast<const char *>(BATCH ? a.bpr[row >> log_m].h3 : a.pr.h3);
+                    for (int k = tp; k < L / 8; k += B::NT)
+                        asm volatile("prefetch.global.L1 [%0];" ::"l"(h3 + k * 128));
+                }
+            }
             B::twiddles_loaded();
             pass_wait();
             pass_release();
@@ -570,13 +632,11 @@ __global__ void __launch_bounds__(Block<Real, LOG_L2, 1, E>::NT, row_min_ctas<Re
                 __syncthreads();  // this row's factor table is complete
 #pragma unroll
                 for (int r = 0; r < E; ++r) {
-                    const int n2 = B::first_pos(tp, r);
-                    if constexpr (B::LIFT) {  // the exact inverse of the PF_TW rotations below
-                        const Lf lo = vec[n2 & 63], hi = vec[64 + (n2 >> 6)];
+                    const Lf lo = tw_thread(r), hi = tw_register(r);
+                    if constexpr (B::LIFT)  // the exact inverse of the PF_TW rotations below
                         v[r] = lift(lift(cscale(v[r], lo.z * hi.z), -hi.x, -hi.y), -lo.x, -lo.y);
-                    } else {
-                        v[r] = cmulc(cmulc(v[r], vec[n2 & 63]), vec[64 + (n2 >> 6)]);
-                    }
+                    else
+                        v[r] = cmulc(cmulc(v[r], lo), hi);
                 }
             }
             // Rows of multi-level plans never transmit (the column pass does).
@@ -624,11 +684,11 @@ __global__ void __launch_bounds__(Block<Real, LOG_L2, 1, E>::NT, row_min_ctas<Re
                 if constexpr (B::LIFT) {
                     // three rotations: the thread's P Q (FP64 product), R[r], h3
                     const double2 *chd = reinterpret_cast<const double2 *>(chp);
-                    const Lf tl = lift_of(cmul(chd[fbase & 63], chd[64 + (fbase >> 6) + NQ / 2]));
+                    const Lf tl = lift_of(SHORT ? thread_chirp : cmul(chd[fbase & 63], chd[64 + (fbase >> 6) + NQ / 2]));
                     const auto rotate = [&](auto cut) {
 #pragma unroll
                         for (int r = 0; r < E; ++r) {
-                            const Lf rr = chp[64 + NQ + r], g = __ldg(h3 + r * B::T + tp);
+                            const Lf rr = chp[RO + r], g = __ldg(h3 + r * B::T + tp);
                             Cx x = cscale(v[r], tl.z * rr.z * g.z);
                             x = lift(lift(lift(x, tl.x, tl.y), rr.x, rr.y), g.x, g.y);
                             v[r] = decltype(cut)::value ? zero_cut(r, x) : x;
@@ -638,11 +698,11 @@ __global__ void __launch_bounds__(Block<Real, LOG_L2, 1, E>::NT, row_min_ctas<Re
                     if (cut_span == 0) rotate(std::false_type{});
                     else rotate(std::true_type{});
                 } else {
-                const Cx tb = cmul(chp[fbase & 63], chp[64 + (fbase >> 6) + NQ / 2]);
+                const Cx tb = SHORT ? thread_chirp : cmul(chp[fbase & 63], chp[64 + (fbase >> 6) + NQ / 2]);
                 const auto multiply = [&](auto cut) {
 #pragma unroll
                     for (int r = 0; r < E; ++r) {
-                        const Cx h = cmul(cmul(tb, chp[64 + NQ + r]), __ldg(h3 + r * B::T + tp));
+                        const Cx h = cmul(cmul(tb, chp[RO + r]), __ldg(h3 + r * B::T + tp));
                         v[r] = decltype(cut)::value ? zero_cut(r, cmul(v[r], h)) : cmul(v[r], h);
                         // a compiler-only barrier per 4 samples: without it all E
                         // h3 loads were issued ahead and held live (the 2^14
@@ -664,6 +724,14 @@ __global__ void __launch_bounds__(Block<Real, LOG_L2, 1, E>::NT, row_min_ctas<Re
             const double2 *tab = a.pr.table + (row << LOG_L2) + tp;
 #pragma unroll
             for (int r = 0; r < E; ++r) v[r] = cvt(cmul(to_f64(v[r]), __ldg(tab + r * B::T)), Cx{});
+        } else if (h_table) {
+#pragma unroll
+            for (int r = 0; r < E; ++r) {
+                const double2 H = hs[r * B::T + tp];
+                const bool zero = H.x == 0.0 && H.y == 0.0;
+                if constexpr (B::LIFT) v[r] = zero ? Cx{} : rot(v[r], lift_of(H));
+                else v[r] = zero ? Cx{} : cmul(v[r], H);
+            }
         } else if (a.pr.has_h || a.pr.has_cut) {
             const int64_t half2 = int64_t(1) << (LOG_L2 - 1);
 #pragma unroll
@@ -681,13 +749,11 @@ __global__ void __launch_bounds__(Block<Real, LOG_L2, 1, E>::NT, row_min_ctas<Re
             if (flags & PF_TW) {
 #pragma unroll
                 for (int r = 0; r < E; ++r) {
-                    const int n2 = B::first_pos(tp, r);
-                    if constexpr (B::LIFT) {
-                        const Lf lo = vec[n2 & 63], hi = vec[64 + (n2 >> 6)];
+                    const Lf lo = tw_thread(r), hi = tw_register(r);
+                    if constexpr (B::LIFT)
                         v[r] = lift(lift(cscale(v[r], lo.z * hi.z), lo.x, lo.y), hi.x, hi.y);
-                    } else {
-                        v[r] = cmul(cmul(v[r], vec[n2 & 63]), vec[64 + (n2 >> 6)]);
-                    }
+                    else
+                        v[r] = cmul(cmul(v[r], lo), hi);
                 }
             } else if (flags & PF_SCALE) {
                 const Real f = Real(a.pr.fac);
@@ -1065,22 +1131,24 @@ static cudaError_t launch_dependent(K kernel, int64_t grid, int threads, size_t 
     return e;
 }
 
-template <int L> constexpr int n_vec() { return 64 + ((L >> 6) > 0 ? (L >> 6) : 1); }
-template <int L, int E> constexpr int n_chirp() { return 64 + ((L >> 6) > 1 ? (L >> 6) : 2) + E; }
-
 template <typename Real, int LG, int E, bool CH, bool TWF, bool BT>
 static cudaError_t row_launch(const PassArgs &a, cudaStream_t s) {
     using B = Block<Real, LG, 1, E>;
     auto k = row_pass_kernel<Real, LG, E, CH, TWF, BT>;
-    const size_t smem = (B::SMEM + 15) / 16 * 16 + 2 * size_t(n_vec<B::L>() + n_chirp<B::L, E>()) * 16;
+    const size_t base = (B::SMEM + 15) / 16 * 16;
+    const size_t smem = base + 2 * size_t(RowTab<LG, E>::NV + RowTab<LG, E>::NCH) * 16;
+    // a single row's transfer function in shared memory (row_threads)
+    constexpr int HT = row_threads<LG, B::NT, CH>();
+    const bool wide = HT > B::NT && a.log_n1 == 0 && a.pr.has_h && !a.pr.table;
+    const size_t smem_h = HT > B::NT && base + size_t(B::L) * 16 > smem ? base + size_t(B::L) * 16 : smem;
     static LaunchSetup setup[LAUNCH_MAX_DEVICES];
     static std::once_flag once[LAUNCH_MAX_DEVICES];
-    const LaunchSetup *st = launch_setup(k, B::NT, smem, smem, setup, once);
+    const LaunchSetup *st = launch_setup(k, B::NT, smem, smem_h, setup, once);
     if (!st) return cudaErrorInvalidDevice;
     if (st->attr != cudaSuccess) return st->attr;
     const int64_t cap = st->cap[0];
     const int64_t rows = a.n >> LG;
-    return launch_dependent(k, rows < cap ? rows : cap, B::NT, smem, s, a.serial != 0, a);
+    return launch_dependent(k, rows < cap ? rows : cap, wide ? HT : B::NT, wide ? smem_h : smem, s, a.serial != 0, a);
 }
 // PF_TWF (rows of three-level plans) takes the TWF variant, for the chirp
 // form and for the per-sample transfer function (exact kernel) alike; rows of
