@@ -1029,22 +1029,33 @@ __device__ __forceinline__ void col_pass(const PassArgs &a) {
     if constexpr (DET) detect_finish(a.det);
 }
 
-// The column kernel. Single-source complex128 tiles of 256 threads take a
-// kernel held to two CTAs per SM: ptxas's default gave the 2^7 outer columns
-// of 2^26 three-level plans 168 registers and one CTA per SM (1028 us per
-// launch), two CTAs at 128 registers and a few spills run 774 us. (Their
-// batched variants keep the default; rsw_sim_run_batch then runs such
-// sources one by one.)
-template <typename Real, int LOG_L1, int C, int E, bool DET = false, bool BATCH = false>
-__global__ void __launch_bounds__(Block<Real, LOG_L1, C, E>::NT) col_pass_kernel(const __grid_constant__ PassArgs a) {
-    col_pass<Real, LOG_L1, C, E, DET, BATCH>(a);
+// The column kernel. CTAs of 256 threads in complex128 and radix 32 are held
+// to two CTAs per SM: ptxas's default gave the 2^7 outer columns of 2^26
+// three-level plans 168 registers and one CTA per SM (1028 us per launch),
+// two CTAs at 128 registers and a few spills run 774 us; the batched form of
+// 2^10 columns with 16 samples per thread takes no spills at 128 registers
+// where it took 255.
+// WIDE: complex128 CTAs of 512 threads (8 samples per thread) at 64 registers,
+// so that two share an SM (a split step over 8 fields of 2^20 25.9 -> 24.6 ps
+// per sample, one field 30.3 -> 28.8). With no more tiles than SMs nothing
+// shares an SM and the few spills only lengthen the pass (2^16: 13.2 against
+// 13.9 us), and a last round that is half empty costs more than the 6 % that
+// sharing gives (2^22: 1024 tiles, 4 rounds of 296 against 7 of 148: 28.3
+// against 27.6 ps): the rule compares the rounds (col_wide).
+template <typename Real, int NT, int E, bool WIDE> constexpr int col_min_ctas() {
+    return WIDE || ((sizeof(Real) == 8 || E == 32) && NT == 256) ? 2 : 1;
 }
-template <typename Real, int LOG_L1, int C, int E> constexpr bool col_two_ctas() {
-    return (sizeof(Real) == 8 || E == 32) && Block<Real, LOG_L1, C, E>::NT == 256;
+static inline bool col_wide(int64_t tiles, int64_t sms) {
+    const int64_t shared = (tiles + 2 * sms - 1) / (2 * sms), plain = (tiles + sms - 1) / sms;
+    return 15 * 2 * shared < 16 * plain;
 }
-template <typename Real, int LOG_L1, int C, int E, bool DET = false, bool BATCH = false>
-__global__ void __launch_bounds__(Block<Real, LOG_L1, C, E>::NT, 2)
-    col_pass_kernel_2cta(const __grid_constant__ PassArgs a) {
+template <typename Real, int NT, int E> constexpr bool col_has_wide() {
+    return sizeof(Real) == 8 && E == 8 && NT == 512;
+}
+template <typename Real, int LOG_L1, int C, int E, bool DET = false, bool BATCH = false, bool WIDE = false>
+__global__ void __launch_bounds__(Block<Real, LOG_L1, C, E>::NT,
+                                  col_min_ctas<Real, Block<Real, LOG_L1, C, E>::NT, E, WIDE>())
+    col_pass_kernel(const __grid_constant__ PassArgs a) {
     col_pass<Real, LOG_L1, C, E, DET, BATCH>(a);
 }
 
@@ -1191,13 +1202,10 @@ template <typename Real> constexpr int col_c32(int log_l) {
 bool encode_col_map(CUtensorMap *map, const void *in, int64_t n, int log_n2, int words_per_sample, int box_w,
                     int box_h);
 
-template <typename Real, int LG, int C, int E, bool DET = false, bool BT = false>
-static cudaError_t col_impl(const PassArgs &a, cudaStream_t s) {
+template <typename Real, int LG, int C, int E, bool DET, bool BT, bool WIDE>
+static cudaError_t col_launch(const PassArgs &a, cudaStream_t s) {
     using B = Block<Real, LG, C, E>;
-    auto k = [] {
-        if constexpr (col_two_ctas<Real, LG, C, E>() && (!BT || sizeof(Real) == 4)) return col_pass_kernel_2cta<Real, LG, C, E, DET, BT>;
-        else return col_pass_kernel<Real, LG, C, E, DET, BT>;
-    }();
+    auto k = col_pass_kernel<Real, LG, C, E, DET, BT, WIDE>;
     // the per-column factor tables only when the pass applies a four-step twiddle
     const size_t plain = B::SMEM;
     const size_t tab = (B::SMEM + 15) / 16 * 16 + ColTab<B::T>::template bytes<C, E, 16>();
@@ -1224,6 +1232,18 @@ static cudaError_t col_impl(const PassArgs &a, cudaStream_t s) {
     b.in_map_ok = a.in && !(a.flags & PF_ONES) && tiles > grid &&
                   encode_col_map(&b.in_map, a.in, a.n, a.log_n2, words, C * words, B::L < 256 ? B::L : 256);
     return launch_dependent(k, grid, B::NT, tables ? tab : plain, s, a.serial != 0, b);
+}
+
+template <typename Real, int LG, int C, int E, bool DET = false, bool BT = false>
+static cudaError_t col_impl(const PassArgs &a, cudaStream_t s) {
+    if constexpr (col_has_wide<Real, Block<Real, LG, C, E>::NT, E>()) {
+        int sms = 0, dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return e;
+        if (col_wide((a.n >> LG) / C, sms)) return col_launch<Real, LG, C, E, DET, BT, true>(a, s);
+    }
+    return col_launch<Real, LG, C, E, DET, BT, false>(a, s);
 }
 
 template <typename Real, int LG, int E> static cudaError_t chirp_impl(void *out, double hi, double lo, cudaStream_t s) {
