@@ -31,16 +31,27 @@ def wavelength_from_energy(energy_ev: float) -> float:
     return H_PLANCK * C_0 / (energy_ev * EV_TO_JOULE)
 
 
-def _torch():
-    import torch
+_torch_module = None
+_raw_stream = None  # torch's current raw stream of a device, where it has that call
 
-    return torch
+
+def _torch():
+    global _torch_module, _raw_stream
+    if _torch_module is None:
+        import torch
+
+        _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        _torch_module = torch
+    return _torch_module
 
 
 def _stream_ptr(stream=None) -> int:
     torch = _torch()
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return int(s.cuda_stream)
+    if stream is not None:
+        return int(stream.cuda_stream)
+    if _raw_stream is not None:  # no stream object per call
+        return _raw_stream(torch.cuda.current_device())
+    return int(torch.cuda.current_stream().cuda_stream)
 
 
 def dtype_code(dtype) -> int:
@@ -102,6 +113,7 @@ class Plan:
         self._lib = L.load()
         self.n = int(n)
         self.code = dtype_code(dtype)
+        self._dtype = torch_dtype(self.code)
         h = C.c_void_p()
         if tuning is None:
             L.check(self._lib.rsw_plan_create(C.byref(h), self.n, self.code))
@@ -120,7 +132,7 @@ class Plan:
 
     @property
     def dtype(self):
-        return torch_dtype(self.code)
+        return self._dtype
 
     def info(self) -> dict:
         n, d, r, c, s = C.c_int64(), C.c_int(), C.c_int(), C.c_int(), C.c_int64()
@@ -129,7 +141,7 @@ class Plan:
                 "scratch_bytes": s.value}
 
     def _check_field(self, t):
-        if t.dtype != self.dtype or t.numel() != self.n:
+        if t.dtype != self._dtype or t.numel() != self.n:
             raise ValueError(f"expected {self.n} values of {self.dtype}, got {t.numel()} of {t.dtype}")
         return _dptr(t)
 
