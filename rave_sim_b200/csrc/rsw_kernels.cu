@@ -51,8 +51,10 @@ cudaError_t launch_row_pass_f64(const PassArgs &a, int e, cudaStream_t s);
 cudaError_t launch_row_pass_f32(const PassArgs &a, int e, cudaStream_t s);
 cudaError_t launch_row_pass_f64_batch(const PassArgs &a, int e, cudaStream_t s);
 cudaError_t launch_row_pass_f32_batch(const PassArgs &a, int e, cudaStream_t s);
-// per-instance transfer functions take the batched kernels
+cudaError_t launch_row_pass_table(const PassArgs &a, bool dbl, cudaStream_t s);
+// table products and per-instance transfer functions have their own kernels
 cudaError_t launch_row_pass(const PassArgs &a, bool dbl, int e, cudaStream_t s) {
+    if (a.pr.table) return e == 16 ? launch_row_pass_table(a, dbl, s) : cudaErrorInvalidValue;
     if (a.bpr) return dbl ? launch_row_pass_f64_batch(a, e, s) : launch_row_pass_f32_batch(a, e, s);
     return dbl ? launch_row_pass_f64(a, e, s) : launch_row_pass_f32(a, e, s);
 }

@@ -467,7 +467,12 @@ template <typename Real, int LOG_L2, int E> struct ChirpTab {
 // the row's own leave (launched so only where the table is used).
 template <int LOG_L2, int NT, bool CHIRP> constexpr int row_threads() { return !CHIRP && LOG_L2 <= 11 ? 256 : NT; }
 
-template <typename Real, int LOG_L2, int E, bool CHIRP, bool TWF = false, bool BATCH = false>
+// TABLE: the spectrum is multiplied by a table (PropArgs::table) in place of a
+// transfer function (with CHIRP set: no per-sample phases). Its own kernel, so
+// that it takes the long rows' register caps: in the per-sample kernel, which
+// needs 220 to 254 registers, the Bluestein rows ran 8 warps on an SM (2^11
+// complex64, 2^22 samples: 46 us).
+template <typename Real, int LOG_L2, int E, bool CHIRP, bool TWF = false, bool BATCH = false, bool TABLE = false>
 __global__ void __launch_bounds__(row_threads<LOG_L2, Block<Real, LOG_L2, 1, E>::NT, CHIRP>(),
                                   row_min_ctas<Real, LOG_L2, E, CHIRP>()) row_pass_kernel(PassArgs a) {
     using B = Block<Real, LOG_L2, 1, E>;
@@ -540,7 +545,7 @@ __global__ void __launch_bounds__(row_threads<LOG_L2, Block<Real, LOG_L2, 1, E>:
         const int64_t kb = digitrev_w(row & ((int64_t(1) << a.log_nb) - 1), a.log_nb, a.rb_nb);
         const int64_t kbase = k1 + (kb << a.log_n1);
         const int64_t tw_k = a.log_nb > 0 ? kb : k1;
-        if (CHIRP && a.pr.has_h) {
+        if (CHIRP && !TABLE && a.pr.has_h) {
             // phase of the row: G kbase^2 + g1 k2s with g1 = 2 M G kbase (turns),
             // M = 2^log_m; P[a] = A exp(2 pi i (G kbase^2 + g1 a)), Q[b] = exp(2 pi i 64 g1 b).
             // k2s = fbase + s_r splits into the thread's part (P[fbase & 63] Q[fbase >> 6],
@@ -601,7 +606,7 @@ __global__ void __launch_bounds__(row_threads<LOG_L2, Block<Real, LOG_L2, 1, E>:
         const auto tw_thread = [&](int r) { return SHORT ? thread_tw : vec[B::first_pos(tp, r) & 63]; };
         const auto tw_register = [&](int r) { return SHORT ? vec[r] : vec[64 + (B::first_pos(tp, r) >> 6)]; };
         if (row == blockIdx.x) {  // what is above does not depend on the preceding kernel
-            if constexpr (SHORT && CHIRP) {
+            if constexpr (SHORT && CHIRP && !TABLE) {
                 // the row's chirp table into L1 (two launches before this one
                 // wrote it: a column pass, which waited for it, lies between)
                 if (a.pr.has_h) {
@@ -663,7 +668,14 @@ __global__ void __launch_bounds__(row_threads<LOG_L2, Block<Real, LOG_L2, 1, E>:
             prefetch_next();
         }
 
-        if constexpr (CHIRP) {
+        if constexpr (TABLE) {
+            const double2 *tab = a.pr.table + (row << LOG_L2) + tp;
+#pragma unroll
+            for (int r = 0; r < E; ++r) {
+                v[r] = cvt(cmul(to_f64(v[r]), __ldg(tab + r * B::T)), Cx{});
+                if (r % 4 == 3) asm volatile("" ::: "memory");  // four entries live at a time
+            }
+        } else if constexpr (CHIRP) {
           if (a.pr.has_h || a.pr.has_cut) {
             // cutoff: k = kbase + k2 2^log_m in [cut_lo, cut_hi)  <=>  k2 in [k2lo, k2hi)
             int k2lo = 0, k2hi = 0;
@@ -765,10 +777,6 @@ __global__ void __launch_bounds__(row_threads<LOG_L2, Block<Real, LOG_L2, 1, E>:
                     if (unsigned((fbase | B::freq_off(r)) - k2lo) < cut_span) v[r] = Cx{};
             }
           }
-        } else if (a.pr.table) {
-            const double2 *tab = a.pr.table + (row << LOG_L2) + tp;
-#pragma unroll
-            for (int r = 0; r < E; ++r) v[r] = cvt(cmul(to_f64(v[r]), __ldg(tab + r * B::T)), Cx{});
         } else if (h_table) {
 #pragma unroll
             for (int r = 0; r < E; ++r) {
@@ -1198,15 +1206,15 @@ static cudaError_t launch_dependent(K kernel, int64_t grid, int threads, size_t 
     return e;
 }
 
-template <typename Real, int LG, int E, bool CH, bool TWF, bool BT>
+template <typename Real, int LG, int E, bool CH, bool TWF, bool BT, bool TABLE = false>
 static cudaError_t row_launch(const PassArgs &a, cudaStream_t s) {
     using B = Block<Real, LG, 1, E>;
-    auto k = row_pass_kernel<Real, LG, E, CH, TWF, BT>;
+    auto k = row_pass_kernel<Real, LG, E, CH, TWF, BT, TABLE>;
     const size_t base = (B::SMEM + 15) / 16 * 16;
     const size_t smem = base + 2 * size_t(RowTab<LG, E>::NV + RowTab<LG, E>::NCH) * 16;
     // a single row's transfer function in shared memory (row_threads)
     constexpr int HT = row_threads<LG, B::NT, CH>();
-    const bool wide = HT > B::NT && a.log_n1 == 0 && a.pr.has_h && !a.pr.table;
+    const bool wide = HT > B::NT && a.log_n1 == 0 && a.pr.has_h;
     const size_t smem_h = HT > B::NT && base + size_t(B::L) * 16 > smem ? base + size_t(B::L) * 16 : smem;
     static LaunchSetup setup[LAUNCH_MAX_DEVICES];
     static std::once_flag once[LAUNCH_MAX_DEVICES];
@@ -1216,6 +1224,13 @@ static cudaError_t row_launch(const PassArgs &a, cudaStream_t s) {
     const int64_t cap = st->cap[0];
     const int64_t rows = a.n >> LG;
     return launch_dependent(k, rows < cap ? rows : cap, wide ? HT : B::NT, wide ? smem_h : smem, s, a.serial != 0, a);
+}
+// table products (Bluestein plans), 16 samples per thread
+template <typename Real, int LG> static cudaError_t row_table(const PassArgs &a, cudaStream_t s) {
+    if constexpr (LG >= 7) {
+        if (a.flags & PF_TWF) return row_launch<Real, LG, 16, true, true, false, true>(a, s);
+    }
+    return row_launch<Real, LG, 16, true, false, false, true>(a, s);
 }
 // PF_TWF (rows of three-level plans) takes the TWF variant, for the chirp
 // form and for the per-sample transfer function (exact kernel) alike; rows of

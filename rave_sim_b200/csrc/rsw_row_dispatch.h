@@ -6,6 +6,26 @@
 #include "rsw_passes.cuh"
 
 namespace rsw {
+// rows of convolution plans (a table product), every length of the per-sample form
+template <typename Real> cudaError_t row_table_dispatch(const PassArgs &a, cudaStream_t s) {
+    switch (a.log_n2) {
+    case 4: return row_table<Real, 4>(a, s);
+    case 5: return row_table<Real, 5>(a, s);
+    case 6: return row_table<Real, 6>(a, s);
+    case 7: return row_table<Real, 7>(a, s);
+    case 8: return row_table<Real, 8>(a, s);
+    case 9: return row_table<Real, 9>(a, s);
+    case 10: return row_table<Real, 10>(a, s);
+    case 11: return row_table<Real, 11>(a, s);
+    case 12: return row_table<Real, 12>(a, s);
+    case 13: return row_table<Real, 13>(a, s);
+    case 14:
+        if constexpr (sizeof(Real) == 4) return row_table<Real, 14>(a, s);
+        [[fallthrough]];
+    default: return cudaErrorInvalidValue;
+    }
+}
+
 // two-level rows (chirp form): 2^7 .. 2^13 (c128) / 2^14 (c64), 16 or 32 elements per thread;
 // single-level rows (per-sample form): 2^4 .. 2^13 / 2^14, 16 elements per thread
 #define RSW_ROW_CASE(R, L) \
@@ -22,10 +42,10 @@ namespace rsw {
     case L: return chirp ? cudaErrorInvalidValue : row_impl<R, L, 16, false, BT>(a, s);
 
 // multi-level rows take the chirp form of the Fresnel kernel; the exact
-// kernel, table products and single-level rows work per sample.
+// kernel and single-level rows work per sample.
 // BT: the batched kernels (chirp form only; the others return an error)
 template <bool BT> cudaError_t row_dispatch_f64(const PassArgs &a, int e, cudaStream_t s) {
-    const bool chirp = a.log_n1 > 0 && !a.pr.exact && !a.pr.table;
+    const bool chirp = a.log_n1 > 0 && !a.pr.exact;
     switch (a.log_n2) {
         RSW_ROW_CASE_S(double, 4) RSW_ROW_CASE_S(double, 5) RSW_ROW_CASE_S(double, 6)
         RSW_ROW_CASE16(double, 7) RSW_ROW_CASE16(double, 8) RSW_ROW_CASE(double, 9)
@@ -34,7 +54,7 @@ template <bool BT> cudaError_t row_dispatch_f64(const PassArgs &a, int e, cudaSt
     }
 }
 template <bool BT> cudaError_t row_dispatch_f32(const PassArgs &a, int e, cudaStream_t s) {
-    const bool chirp = a.log_n1 > 0 && !a.pr.exact && !a.pr.table;
+    const bool chirp = a.log_n1 > 0 && !a.pr.exact;
     switch (a.log_n2) {
         RSW_ROW_CASE_S(float, 4) RSW_ROW_CASE_S(float, 5) RSW_ROW_CASE_S(float, 6) RSW_ROW_CASE16(float, 7)
         RSW_ROW_CASE16(float, 8) RSW_ROW_CASE(float, 9) RSW_ROW_CASE(float, 10) RSW_ROW_CASE8(float, 11)
