@@ -1224,20 +1224,31 @@ static cudaError_t to_spec(const rsw_plan_s *p, const void *nat, void *spec, cud
     return launch_natural_to_spec(nat, spec, p->n, spec_levels(p), p->dbl(), s);
 }
 
+// Natural-order FFTs of single rows, n a multiple of the plan's length: one
+// pass, which reads or writes the spectrum in natural order (in == out allowed:
+// a row is in registers before any of it is written).
+static rsw_status single_fft(const rsw_plan_s *p, const void *in, void *out, int64_t n, bool inverse, cudaStream_t s) {
+    PassArgs a = base_args(p);
+    a.n = n;
+    a.in = in;
+    a.out = out;
+    a.flags = PF_NAT | (inverse ? PF_SPEC_IN | PF_INV | PF_SCALE : PF_FWD);
+    return run_row(p, a, s);
+}
+
 rsw_status rsw_fft_forward(rsw_plan p, const void *in, void *out, void *stream) {
     if (!p || !in || !out) return fail(RSW_ERR_INVALID, "NULL argument");
     cudaStream_t s = (cudaStream_t)stream;
     if (p->blue) return blue_transform(p, in, out, false, s);
+    if (p->log_n1 == 0) return single_fft(p, in, out, p->n, false, s);
     CHECK(need_scratch(p));
     PassArgs a = base_args(p);
     a.in = in;
     a.out = p->scratch.p;
-    if (p->log_n1 > 0) {
-        a.flags = PF_FWD | PF_TW;
-        CHECK(run_col(p, a, s));
-        a.in = p->scratch.p;
-        if (p->three()) CHECK(run_mid(p, a, true, s));
-    }
+    a.flags = PF_FWD | PF_TW;
+    CHECK(run_col(p, a, s));
+    a.in = p->scratch.p;
+    if (p->three()) CHECK(run_mid(p, a, true, s));
     PassArgs r = row_level(p, a);
     r.flags = PF_FWD | row_tw(p, true, false);
     CHECK(run_row(p, r, s));
@@ -1250,26 +1261,21 @@ rsw_status rsw_fft_inverse(rsw_plan p, const void *in, void *out, void *stream) 
     if (!p || !in || !out) return fail(RSW_ERR_INVALID, "NULL argument");
     cudaStream_t s = (cudaStream_t)stream;
     if (p->blue) return blue_transform(p, in, out, true, s);
+    if (p->log_n1 == 0) return single_fft(p, in, out, p->n, true, s);
     CHECK(need_scratch(p));
     cudaError_t e = to_spec(p, in, p->scratch.p, s);
     if (e != cudaSuccess) return fail(RSW_ERR_CUDA, "reorder: %s", cudaGetErrorString(e));
     PassArgs a = base_args(p);
     a.in = p->scratch.p;
-    if (p->log_n1 > 0) {
-        PassArgs r = row_level(p, a);
-        r.out = p->scratch.p;
-        r.flags = PF_SPEC_IN | PF_INV | row_tw(p, false, true);
-        CHECK(run_row(p, r, s));
-        a.out = p->scratch.p;
-        if (p->three()) CHECK(run_mid(p, a, false, s));
-        a.out = out;
-        a.flags = col_inv(p);
-        CHECK(run_col(p, a, s));
-    } else {
-        a.out = out;
-        a.flags = PF_SPEC_IN | PF_INV | PF_SCALE;
-        CHECK(run_row(p, a, s));
-    }
+    PassArgs r = row_level(p, a);
+    r.out = p->scratch.p;
+    r.flags = PF_SPEC_IN | PF_INV | row_tw(p, false, true);
+    CHECK(run_row(p, r, s));
+    a.out = p->scratch.p;
+    if (p->three()) CHECK(run_mid(p, a, false, s));
+    a.out = out;
+    a.flags = col_inv(p);
+    CHECK(run_col(p, a, s));
     return RSW_OK;
 }
 
@@ -1282,18 +1288,17 @@ rsw_status rsw_fft_inverse(rsw_plan p, const void *in, void *out, void *stream) 
 static rsw_status fft_batch(rsw_plan_s *p, const void *in, void *out, int64_t count, bool inverse, void *work,
                             cudaStream_t s) {
     const int64_t total = count * p->n;
+    if (p->log_n1 == 0) return single_fft(p, in, out, total, inverse, s);
     PassArgs a = base_args(p);
     a.n = total;
     cudaError_t e;
     if (!inverse) {
         a.in = in;
         a.out = work;
-        if (p->log_n1 > 0) {
-            a.flags = PF_FWD | PF_TW;
-            CHECK(run_col(p, a, s));
-            a.in = work;
-            if (p->three()) CHECK(run_mid(p, a, true, s));
-        }
+        a.flags = PF_FWD | PF_TW;
+        CHECK(run_col(p, a, s));
+        a.in = work;
+        if (p->three()) CHECK(run_mid(p, a, true, s));
         PassArgs r = row_level(p, a);
         r.flags = PF_FWD | row_tw(p, true, false);
         CHECK(run_row(p, r, s));
@@ -1304,22 +1309,15 @@ static rsw_status fft_batch(rsw_plan_s *p, const void *in, void *out, int64_t co
     e = launch_natural_to_spec(in, work, total, spec_levels(p), p->dbl(), s);
     if (e != cudaSuccess) return fail(RSW_ERR_CUDA, "reorder: %s", cudaGetErrorString(e));
     a.in = work;
-    if (p->log_n1 > 0) {
-        PassArgs r = row_level(p, a);
-        r.out = work;
-        r.flags = PF_SPEC_IN | PF_INV | row_tw(p, false, true);
-        CHECK(run_row(p, r, s));
-        a.out = work;
-        if (p->three()) CHECK(run_mid(p, a, false, s));
-        a.out = out;
-        a.flags = col_inv(p);
-        CHECK(run_col(p, a, s));
-    } else {
-        a.out = out;
-        a.flags = PF_SPEC_IN | PF_INV | PF_SCALE;
-        CHECK(run_row(p, a, s));
-    }
-    return RSW_OK;
+    PassArgs r = row_level(p, a);
+    r.out = work;
+    r.flags = PF_SPEC_IN | PF_INV | row_tw(p, false, true);
+    CHECK(run_row(p, r, s));
+    a.out = work;
+    if (p->three()) CHECK(run_mid(p, a, false, s));
+    a.out = out;
+    a.flags = col_inv(p);
+    return run_col(p, a, s);
 }
 
 // The four-step of big-fourier's out-of-core fft (big-fourier/src/bfft.rs:27-100):
@@ -1422,6 +1420,20 @@ rsw_status rsw_propagate(rsw_plan p, void *u, void *U, double dx, double wl, dou
     }
     a.in = u;
     a.out = u;
+    if (!two && U) {
+        // one row: the transfer function's pass leaves the spectrum in U in
+        // natural order, and the inverse reads it there
+        a.in = skip_fft ? U : u;
+        a.out = U;
+        a.flags = PF_NAT | (skip_fft ? PF_SPEC_IN : PF_FWD);
+        CHECK(run_row(p, a, s));
+        a.pr.has_h = 0;
+        a.pr.has_cut = 0;
+        a.in = U;
+        a.out = u;
+        a.flags = PF_NAT | PF_SPEC_IN | PF_INV | PF_SCALE;
+        return run_row(p, a, s);
+    }
     // 1. spectrum of u in the internal layout, in place in u
     if (skip_fft) {
         cudaError_t e = to_spec(p, U, u, s);

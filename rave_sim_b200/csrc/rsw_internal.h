@@ -78,6 +78,7 @@ enum PassFlags : int {
     PF_TWI = 128,     // column: before the inverse, conj(W_M^(n2 k1)) * tw_scale
     PF_TWF = 256,     // row: before the forward, W_M^(n2 tw_k) (the conjugate of PF_TW's factor)
     PF_NOSTORE = 512, // column detection pass: bin the field only, do not write it
+    PF_NAT = 1024,    // single-level row: the spectrum read or written is in natural order
 };
 
 // Per-instance values of a batched pass: several sources with the same
