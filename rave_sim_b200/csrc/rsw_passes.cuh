@@ -1196,8 +1196,11 @@ static const LaunchSetup *launch_setup(K kernel, int threads, size_t smem, size_
 // launch with programmatic dependent launch (pass_wait): the CTAs of a short
 // pass load their twiddles and build their factor tables while the pass
 // before it finishes. A split step of 2^16 complex128 samples (two launches)
-// 22.9 -> 13.4 us, 2^14 complex64 22.9 -> 10.9, 2^20 complex128 35.2 -> 29.7;
-// no change from 2^24 on.
+// 22.9 -> 13.4 us, 2^14 complex64 22.9 -> 10.9, 2^20 complex128 35.2 -> 29.7.
+// Passes over 512 MB and more launch serially (pass_serial): their start-up is
+// hidden anyway, and CTAs that arrive while the last ones finish cost more
+// than they save (a sample run at 2^26 complex64 72.9 against 71.5 ms, 8
+// sources 567 against 548; at 2^24 15.3 against 15.6 the other way).
 template <typename K, typename... Args>
 static cudaError_t launch_dependent(K kernel, int64_t grid, int threads, size_t smem, cudaStream_t s, bool serial,
                                     const Args &...args) {
@@ -1214,6 +1217,10 @@ static cudaError_t launch_dependent(K kernel, int64_t grid, int threads, size_t 
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
     if (e == cudaSuccess) count_launch();
     return e;
+}
+
+static inline bool pass_serial(const PassArgs &a, size_t elem) {
+    return a.serial || a.n >= (int64_t(1) << 29) / int64_t(elem);
 }
 
 template <typename Real, int LG, int E, bool CH, bool TWF, bool BT, bool TABLE = false>
@@ -1233,7 +1240,8 @@ static cudaError_t row_launch(const PassArgs &a, cudaStream_t s) {
     if (st->attr != cudaSuccess) return st->attr;
     const int64_t cap = st->cap[0];
     const int64_t rows = a.n >> LG;
-    return launch_dependent(k, rows < cap ? rows : cap, wide ? HT : B::NT, wide ? smem_h : smem, s, a.serial != 0, a);
+    return launch_dependent(k, rows < cap ? rows : cap, wide ? HT : B::NT, wide ? smem_h : smem, s, pass_serial(a, sizeof(typename B::Cx)),
+                            a);
 }
 // table products (Bluestein plans), 16 samples per thread
 template <typename Real, int LG> static cudaError_t row_table(const PassArgs &a, cudaStream_t s) {
@@ -1312,7 +1320,7 @@ static cudaError_t col_launch(const PassArgs &a, cudaStream_t s) {
     constexpr int words = int(sizeof(typename B::Cx) / 8);
     b.in_map_ok = a.in && !(a.flags & PF_ONES) && tiles > grid &&
                   encode_col_map(&b.in_map, a.in, a.n, a.log_n2, words, C * words, B::L < 256 ? B::L : 256);
-    return launch_dependent(k, grid, B::NT, tables ? tab : plain, s, a.serial != 0, b);
+    return launch_dependent(k, grid, B::NT, tables ? tab : plain, s, pass_serial(a, sizeof(typename B::Cx)), b);
 }
 
 template <typename Real, int LG, int C, int E, bool DET = false, bool BT = false>
