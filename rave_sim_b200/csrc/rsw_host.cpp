@@ -572,7 +572,8 @@ static rsw_status plan_split(int64_t n, int dtype, int *log_n, int *l1, int *lb,
 // columns of 2^10: 40 us a split step against 49 with 8 per thread and 4
 // columns), and so do the outer columns of three-level plans (2^26 complex128
 // 2.53 against 2.59 ms). Everything else takes 16.
-// RSW_ROW_E / RSW_COL_E (8, 16 or 32) override the choice (tuning sweeps).
+// RSW_ROW_E / RSW_COL_E (8, 16 or 32) override the choice (tuning sweeps) for
+// the levels that have such a kernel.
 static int env_int(const char *name, int dflt) {
     const char *v = std::getenv(name);
     return v && *v ? std::atoi(v) : dflt;
@@ -616,13 +617,11 @@ static rsw_status choose_tuning(rsw_plan_s *p, const rsw_tuning *t) {
         if (t->mid_e) p->mid_e = t->mid_e;
         return RSW_OK;
     }
+    // where a kernel exists; the default elsewhere
     const int re = env_int("RSW_ROW_E", 0), ce = env_int("RSW_COL_E", 0);
-    if ((re == 16 || re == 32) && p->log_nr >= 9) p->row_e = re;
-    p->row_tuned = re == 8 || re == 16 || re == 32;
-    if (ce == 16 || (ce == 32 && p->log_n1 >= 9)) p->col_e = ce;
-    // 8 samples per thread: multi-level rows of 2^11..2^13, columns of 2^8..2^11
-    if (re == 8 && p->log_n1 > 0 && p->log_nr >= 11 && p->log_nr <= 13) p->row_e = 8;
-    if (ce == 8 && p->log_n1 >= 8 && p->log_n1 <= 11) p->col_e = 8;
+    p->row_tuned = re && row_e_ok(p->log_nr, l1 > 0, re);
+    if (p->row_tuned) p->row_e = re;
+    if (ce && l1 > 0 && col_e_ok(l1, ce, c128)) p->col_e = ce;
     return RSW_OK;
 }
 

@@ -27,19 +27,21 @@ template <typename Real> cudaError_t row_table_dispatch(const PassArgs &a, cudaS
 }
 
 // two-level rows (chirp form): 2^7 .. 2^13 (c128) / 2^14 (c64), 16 or 32 elements per thread;
-// single-level rows (per-sample form): 2^4 .. 2^13 / 2^14, 16 elements per thread
+// single-level rows (per-sample form): 2^4 .. 2^13 / 2^14, 16 elements per thread. A count that a
+// length has no kernel for is an error: the plan's tables are laid out for it.
+#define RSW_ROW_E(R, L, E, CH) (e == E ? row_impl<R, L, E, CH, BT>(a, s) : cudaErrorInvalidValue)
 #define RSW_ROW_CASE(R, L) \
-    case L: return chirp ? (e == 32 ? row_impl<R, L, 32, true, BT>(a, s) : row_impl<R, L, 16, true, BT>(a, s)) \
-                         : row_impl<R, L, 16, false, BT>(a, s);
+    case L: return chirp && e == 32 ? row_impl<R, L, 32, true, BT>(a, s) \
+                                    : chirp ? RSW_ROW_E(R, L, 16, true) : RSW_ROW_E(R, L, 16, false);
 #define RSW_ROW_CASE16(R, L) \
-    case L: return chirp ? row_impl<R, L, 16, true, BT>(a, s) : row_impl<R, L, 16, false, BT>(a, s);
+    case L: return chirp ? RSW_ROW_E(R, L, 16, true) : RSW_ROW_E(R, L, 16, false);
 // rows with 8 samples per thread (radix-8 stages, twice the threads)
 #define RSW_ROW_CASE8(R, L) \
-    case L: return chirp ? (e == 8 ? row_impl<R, L, 8, true, BT>(a, s) \
-                                   : e == 32 ? row_impl<R, L, 32, true, BT>(a, s) : row_impl<R, L, 16, true, BT>(a, s)) \
-                         : row_impl<R, L, 16, false, BT>(a, s);
+    case L: return chirp && e == 8 ? row_impl<R, L, 8, true, BT>(a, s) \
+                   : chirp && e == 32 ? row_impl<R, L, 32, true, BT>(a, s) \
+                                      : chirp ? RSW_ROW_E(R, L, 16, true) : RSW_ROW_E(R, L, 16, false);
 #define RSW_ROW_CASE_S(R, L) \
-    case L: return chirp ? cudaErrorInvalidValue : row_impl<R, L, 16, false, BT>(a, s);
+    case L: return chirp ? cudaErrorInvalidValue : RSW_ROW_E(R, L, 16, false);
 
 // multi-level rows take the chirp form of the Fresnel kernel; the exact
 // kernel and single-level rows work per sample.
@@ -62,6 +64,7 @@ template <bool BT> cudaError_t row_dispatch_f32(const PassArgs &a, int e, cudaSt
     default: return cudaErrorInvalidValue;
     }
 }
+#undef RSW_ROW_E
 #undef RSW_ROW_CASE
 #undef RSW_ROW_CASE16
 #undef RSW_ROW_CASE8
