@@ -629,8 +629,11 @@ __global__ void __launch_bounds__(row_threads<LOG_L2, Block<Real, LOG_L2, 1, E>:
             pass_wait();
             pass_release();
             __syncthreads();
-        } else if constexpr (B::NS == 1) {
-            __syncthreads();  // no barrier inside a one-stage transform
+        } else if (B::NS == 1 || (CHIRP && !TABLE && (flags & PF_SPEC_IN) && a.pr.has_h)) {
+            // the tables above are complete: no barrier inside a one-stage
+            // transform, and a given spectrum meets the chirp factors without
+            // the forward transform's barriers in between
+            __syncthreads();
         }
         const Cx *gin = static_cast<const Cx *>(a.in) + (row << LOG_L2);
         Cx *gout = static_cast<Cx *>(a.out) + (row << LOG_L2);
