@@ -1101,10 +1101,11 @@ rsw_status rsw_autotune_batch(int64_t n, int dtype, int64_t fields, int reps, rs
         for (int l1 = 4; l1 <= col_max; ++l1) {
             const int lb = lg - row_max - l1;
             if (lb < 4 || lb > col_max) continue;
-            for (int ce : {16, 8})
-                for (int me : {16, 8})
-                    if (col_e_ok(l1, ce, c128) && col_e_ok(lb, me, c128))
-                        cands.push_back(rsw_tuning{3, l1, lb, 16, ce, me});
+            for (int re : {16, 32})
+                for (int ce : {16, 8})
+                    for (int me : {16, 8})
+                        if (row_e_ok(row_max, true, re) && col_e_ok(l1, ce, c128) && col_e_ok(lb, me, c128))
+                            cands.push_back(rsw_tuning{3, l1, lb, re, ce, me});
         }
     }
     cudaStream_t s = (cudaStream_t)stream;
