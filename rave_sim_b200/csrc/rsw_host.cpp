@@ -526,15 +526,16 @@ static rsw_status plan_split(int64_t n, int dtype, int *log_n, int *l1, int *lb,
         if (lg > row_max + 2 * col_max)
             return fail(RSW_ERR_UNSUPPORTED, "N = 2^%d exceeds the three-level limit 2^%d for this dtype", lg,
                         row_max + 2 * col_max);
-        // outer columns of 2^8 and the rest in the middle while that stays
-        // short (split step at 2^26 complex128: 2.53 ms against 2.59 for
-        // columns of 2^9; 2^27 complex128 5.03 against 5.61 for 2^10, complex64
-        // 2.98 against 3.06 for 2^9); beyond, long outer columns (the pass
-        // with the transmission and the factor tables, which amortise over
-        // the column length) and the rest in the middle, at least 2^4
+        // complex128: outer columns of 2^8 and the rest in the middle while
+        // that stays short (split step at 2^26 2.48 ms against 2.57 for columns
+        // of 2^9, 2^27 4.98 against 5.44 for 2^10). Elsewhere long outer columns
+        // (the pass with the transmission and the factor tables, which amortise
+        // over the column length) and the rest in the middle, at least 2^4:
+        // complex64 2^27 in columns of 2^9 2.97 ms against 3.52 for 2^8, 2^28 in
+        // columns of 2^10 5.75 against 7.00, a propagation 6.00 against 7.26
         const int rest = lg - row_max;
         *lr = row_max;
-        *l1 = rest <= 14 ? 8 : std::min(std::min(col_max, 11), rest - 4);
+        *l1 = dtype == RSW_C128 && rest <= 14 ? 8 : std::min(std::min(col_max, 11), rest - 4);
         *lb = rest - *l1;
         if (*lb > col_max) {
             *lb = col_max;

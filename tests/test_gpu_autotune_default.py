@@ -23,3 +23,14 @@ def test_default_is_tried(monkeypatch, dt, lg):
     p.close()
     tried = autotune.tune(1 << lg, dt, reps=1, save=False, register_result=False)["tried"]
     assert default in [t for t, _ in tried]
+
+
+# the fastest splits by measurement (complex64 outer columns of 2^8 run a
+# split step 18 % and 22 % slower at 2^27 and 2^28, complex128 ones of 2^9
+# and 2^10 4 % and 9 % slower at 2^26 and 2^27)
+@pytest.mark.parametrize("dt,lg,split", [("c8", 27, (9, 4)), ("c8", 28, (10, 4)), ("c16", 26, (8, 5)), ("c16", 27, (8, 6))])
+def test_default_three_level_split(monkeypatch, dt, lg, split):
+    for v in ("RSW_SPLIT", "RSW_SPLIT3", "RSW_ROW_E", "RSW_COL_E"):
+        monkeypatch.delenv(v, raising=False)
+    t = autotune.plan_tuning(rsw.Plan(1 << lg, dt))
+    assert (t["levels"], t["log_rows"], t["log_mid"]) == (3, *split)
