@@ -325,9 +325,13 @@ struct rsw_plan_s {
     int log_nb = 0, log_nr = 0;  // N2 = Nb * Nr: middle level (0: two-level) and row-kernel length
     int device = 0;
     int row_e = 16, col_e = 16, mid_e = 16;  // elements per thread of the row / column / middle kernels
-    bool row_tuned = false;                  // row_e was asked for (a tuning, RSW_ROW_E)
     int prop_mode = RSW_PROP_FRESNEL;        // transfer function of propagate and of simulations
     DevBuf tw_row, tw_col, tw_mid, tw4_lo, tw4_hi, tw4b_lo, tw4b_hi;
+    // Rows whose default is not 16 samples per thread: the count and the table
+    // of the other propagator (the exact one has kernels of 16 only), exchanged
+    // with row_e and tw_row by rsw_plan_set_propagator; 0: both run row_e
+    int row_e_other = 0;
+    DevBuf tw_row_other;
     int tw4_shift = 0, tw4b_shift = 0;
     DevBuf scratch;                                       // N samples, for the natural-order APIs
     DevBuf det_bounds, det_cos, det_r;                    // cached detector geometry
@@ -437,6 +441,8 @@ static rsw_status four_step_tables(int log_m, DevBuf &lo_buf, DevBuf &hi_buf, in
 
 template <typename T> static rsw_status plan_tables(rsw_plan_s *p) {
     CHECK(p->tw_row.upload(block_twiddles<T>(p->log_nr, digit_bits(p->row_e))));
+    if (p->row_e_other)
+        CHECK(p->tw_row_other.upload(block_twiddles<T>(p->log_nr, digit_bits(p->row_e_other))));
     if (p->log_n1 > 0) {
         CHECK(p->tw_col.upload(block_twiddles<T>(p->log_n1, digit_bits(p->col_e))));
         CHECK(four_step_tables(p->log_n, p->tw4_lo, p->tw4_hi, &p->tw4_shift));
@@ -596,7 +602,9 @@ static rsw_status choose_tuning(rsw_plan_s *p, const rsw_tuning *t) {
     // complex64 rows of 2^14 in radix 32: three stages and two exchanges per
     // direction in place of four and three (split step at 2^26 1.32 -> 1.27
     // ms, 2^25 548 -> 536 us; at 2^13 the 32 warps of radix 16 are as fast)
-    p->row_e = p->dtype == RSW_C64 && p->log_n1 > 0 && p->log_nr == 14 ? 32 : pick(p->log_nr, 16);
+    const int row_dflt = p->dtype == RSW_C64 && p->log_n1 > 0 && p->log_nr == 14 ? 32 : pick(p->log_nr, 16);
+    p->row_e = row_dflt;
+    if (row_dflt != 16) p->row_e_other = 16;
     const bool c128 = p->dtype == RSW_C128;
     const int l1 = p->log_n1;
     p->col_e = (c128 && l1 >= 8 && l1 <= 12 && p->log_nb == 0) || (!c128 && l1 == 9) ? 8 : pick(l1, 16);
@@ -613,15 +621,17 @@ static rsw_status choose_tuning(rsw_plan_s *p, const rsw_tuning *t) {
             return fail(RSW_ERR_INVALID, "tuning: no middle kernel of 2^%d with %d samples per thread", p->log_nb,
                         t->mid_e);
         if (t->row_e) p->row_e = t->row_e;
-        p->row_tuned = t->row_e != 0;
+        if (p->row_e != row_dflt) p->row_e_other = 0;
         if (t->col_e) p->col_e = t->col_e;
         if (t->mid_e) p->mid_e = t->mid_e;
         return RSW_OK;
     }
     // where a kernel exists; the default elsewhere
     const int re = env_int("RSW_ROW_E", 0), ce = env_int("RSW_COL_E", 0);
-    p->row_tuned = re && row_e_ok(p->log_nr, l1 > 0, re);
-    if (p->row_tuned) p->row_e = re;
+    if (re && row_e_ok(p->log_nr, l1 > 0, re)) {
+        p->row_e = re;
+        p->row_e_other = 0;
+    }
     if (ce && l1 > 0 && col_e_ok(l1, ce, c128)) p->col_e = ce;
     return RSW_OK;
 }
@@ -1200,17 +1210,15 @@ rsw_status rsw_plan_info(rsw_plan p, int64_t *n, int *dtype, int *log_rows, int 
 rsw_status rsw_plan_set_propagator(rsw_plan p, int mode) {
     if (!p) return fail(RSW_ERR_INVALID, "plan is NULL");
     if (mode != RSW_PROP_FRESNEL && mode != RSW_PROP_EXACT) return fail(RSW_ERR_INVALID, "unknown propagator %d", mode);
-    // the exact kernel runs the per-sample row kernels (16 samples per
-    // thread): a plan whose rows took another count by default changes over
-    if (mode == RSW_PROP_EXACT && p->log_n1 > 0 && p->row_e != 16) {
-        if (p->row_tuned)
-            return fail(RSW_ERR_UNSUPPORTED, "the exact propagator needs rows of 16 samples per thread");
-        DevBuf tw;
-        CHECK(p->dbl() ? tw.upload(block_twiddles<double>(p->log_nr, digit_bits(16)))
-                       : tw.upload(block_twiddles<float>(p->log_nr, digit_bits(16))));
-        CU(cudaDeviceSynchronize());  // the old table's readers
-        p->tw_row = std::move(tw);
-        p->row_e = 16;
+    // The exact kernel runs the per-sample row kernels (16 samples per thread).
+    // Rows of another count by default change over, and back: both tables are
+    // the plan's from its creation, so no call in flight loses its own. A count
+    // that was asked for (RSW_ROW_E, a tuning other than the default) stays.
+    if (mode == RSW_PROP_EXACT && p->log_n1 > 0 && p->row_e != 16 && !p->row_e_other)
+        return fail(RSW_ERR_UNSUPPORTED, "the exact propagator needs rows of 16 samples per thread");
+    if (mode != p->prop_mode && p->row_e_other) {
+        std::swap(p->row_e, p->row_e_other);
+        std::swap(p->tw_row, p->tw_row_other);
     }
     p->prop_mode = mode;
     return RSW_OK;
