@@ -2631,25 +2631,6 @@ rsw_status rsw_sim_run(rsw_sim S, const rsw_source *src, const rsw_source_run *r
 
 }  // extern "C"
 
-// Whether the batched column kernel of the plan's transmitting pass holds as
-// many CTAs per SM as the plain one. Its per-instance factors take registers
-// that the plain kernel does not need; where that costs resident CTAs (some
-// complex128 column shapes of 64 to 256 threads), a batch is slower than the
-// same sources one after the other (2^26 complex128, three levels with
-// columns of 2^7: 24.1 against 27.5 G samples*steps/s on B200).
-static bool batch_keeps_occupancy(const rsw_plan_s *P) {
-    PassArgs a = base_args(P);
-    a.flags = PF_FWD | PF_INV | PF_TW | PF_TRANS | (P->three() ? PF_TWI : 0);
-    int64_t plain = 0, batched = 0;
-    a.resident = &plain;
-    if (launch_col_pass(a, P->dbl(), P->col_e, nullptr) != cudaSuccess) return false;
-    BatchTrans dummy{};
-    a.btr = &dummy;
-    a.resident = &batched;
-    if (launch_col_pass(a, P->dbl(), P->col_e, nullptr) != cudaSuccess) return false;
-    return batched >= plain;
-}
-
 extern "C" {
 
 // Sources per lockstep chunk: as many as fit, with their batch buffers, in
@@ -2771,8 +2752,7 @@ rsw_status rsw_sim_run_batch(rsw_sim S, const rsw_source *srcs, int64_t n_source
     // sources one after the other, with the same results
     const bool lockstep = count > 1 && P->log_n1 > 0 && !P->blue && P->prop_mode == RSW_PROP_FRESNEL &&
                           S->hist_dz == 0.0 && S->keypoints.empty() && S->final_fields.empty() &&
-                          !S->els.empty() && S->geom.n_pix > 0 && same_kind &&
-                          batch_keeps_occupancy(P);
+                          !S->els.empty() && S->geom.n_pix > 0 && same_kind;
     // consecutive chunks keep the order in which every (phase step, pixel)
     // accumulator receives the sources
     const int64_t chunk = lockstep ? batch_chunk(S, count) : 1;

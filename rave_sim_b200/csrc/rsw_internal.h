@@ -156,9 +156,6 @@ struct PassArgs {
     // column pass, per instance of the batch; row pass, likewise
     const BatchTrans *btr;
     const BatchProp *bpr;
-    // column pass: when set, the launch functions store the kernel's resident
-    // CTAs on the current device here and launch nothing
-    int64_t *resident;
     // launch after the preceding kernel has completed: its tables were written
     // in this stream (programmatic dependent launch reads them before)
     int serial;

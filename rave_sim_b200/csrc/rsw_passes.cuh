@@ -933,8 +933,8 @@ __device__ __forceinline__ void detect_finish(const DetectArgs &d) {
 // PF_NOSTORE; the last CTA finishes the detector row (detect_finish).
 // BATCH: per-instance transmission factors (a.btr), a separate kernel. Its
 // factors live in registers where the plain kernel reads them from the
-// parameter bank, so some complex128 shapes hold fewer CTAs per SM
-// (col_resident; the host then runs such sources one after the other).
+// parameter bank; within the register caps (col_min_ctas) every shape still
+// holds as many CTAs per SM as the plain one.
 template <typename Real, int LOG_L1, int C, int E, bool DET, bool BATCH>
 __device__ __forceinline__ void col_pass(const PassArgs &a) {
     using B = Block<Real, LOG_L1, C, E>;
@@ -1308,10 +1308,6 @@ static cudaError_t col_launch(const PassArgs &a, cudaStream_t s) {
     if (st->attr != cudaSuccess) return st->attr;
     const bool tables = a.flags & (PF_TW | PF_TWI);
     const int64_t cap = tables ? st->cap[0] : st->cap[1];
-    if (a.resident) {  // a query: the resident CTAs per device, no launch
-        *a.resident = cap;
-        return cudaSuccess;
-    }
     const int64_t tiles = (a.n >> LG) / C;
     if ((int64_t(1) << a.log_n2) < C) return cudaErrorInvalidValue;  // fewer columns per batch than a tile
     int64_t grid = tiles < cap ? tiles : cap;
