@@ -28,8 +28,8 @@
 // Twiddles W_{RS}^{jq} of stage s live in shared memory, loaded once per CTA:
 // a direct table [(q-1)*S + j] for strides S <= 128 (512 for complex64),
 // otherwise two factors W^{(j mod 64) q} * W^{64 (j div 64) q} of 64 and S/64
-// entries per q. FP64 butterflies may take only W^j from the tables and form
-// the other powers as a running product (running()).
+// entries per q. FP64 butterflies may take only some powers from the tables
+// and form the others as products (by_powers()).
 //
 // Complex64 blocks rotate by lifting instead of complex multiplication: a
 // rotation by theta is three shears xr += a xi; xi += b xr; xr += a xi with
@@ -408,15 +408,36 @@ struct Block : Radix<LOG_L, E_, direct_max_ls(2 * sizeof(Real), LOG_L, digit_bit
         }
     }
 
-    // FP64 twiddles as the running product W^(jq) = W^(j(q-1)) W^j (error
-    // below R ulp): one table lookup per butterfly instead of R - 1. For
+    // FP64 twiddles W^(jq) as products of a few looked-up powers (powers): q = 1
+    // and every multiple of 4 from the tables, q = 2 too in radix 16 and 32
+    // (radix 8 squares the first), the others by at most two products. For
     // factored stages this takes as many complex products as the two-factor
-    // lookups. Radix-8 blocks of 2^10 and more (the 1024-thread complex128
-    // column kernels, held back by shared-memory instruction issue) also
-    // trade the direct lookups for R - 2 products: 7 % faster at 2^11.
-    // complex64 keeps the lookups.
-    template <int s> static constexpr bool running() {
+    // lookups, and 5 lookups of two entries per radix-16 butterfly in place of
+    // 15. Radix-8 blocks of 2^10 and more (the 1024-thread complex128 column
+    // kernels, held back by shared-memory instruction issue) also trade 5 of
+    // their 7 direct lookups for products. A running product W^(j(q-1)) W^j
+    // needs one lookup only, but multiplies that entry's rounding by q: an rms
+    // error of 4.9e-16 per radix-16 factor and 2.5e-16 per radix-8 one, against
+    // 0.9e-16 and 1.2e-16. complex64 keeps the lookups.
+    template <int s> static constexpr bool by_powers() {
         return sizeof(Real) == 8 && (!Rx::direct(s) || (E == 8 && LOG_L >= 10));
+    }
+    // apply(q, W^(jq)) for q = 1 .. R - 1
+    template <int s, typename F> __device__ static __forceinline__ void powers(const Tw *tw, int j, F apply) {
+        constexpr int R = 1 << Rx::lr(s);
+        const Cx w1 = twid<s>(tw, j, 1), w2 = R == 8 ? cmul(w1, w1) : twid<s>(tw, j, 2);
+        apply(1, w1);
+        apply(2, w2);
+        apply(3, cmul(w2, w1));
+#pragma unroll
+        for (int q = 4; q < R; q += 4) {
+            const Cx w = twid<s>(tw, j, q);
+            apply(q, w);
+            apply(q + 1, cmul(w, w1));
+            const Cx v = cmul(w, w2);
+            apply(q + 2, v);
+            apply(q + 3, cmul(v, w1));
+        }
     }
 
     // forward stage s: natural in -> radix-R DFT -> bit-reversed out, twiddled
@@ -428,15 +449,8 @@ struct Block : Radix<LOG_L, E_, direct_max_ls(2 * sizeof(Real), LOG_L, digit_bit
             net_dif<R, -1>(v + i * R);
             if constexpr (s < NS - 1) {
                 const int j = Rx::beta(s, tp, i) & ((1 << LSS) - 1);
-                if constexpr (running<s>()) {
-                    const Cx w1 = twid<s>(tw, j, 1);
-                    Cx w = w1;
-#pragma unroll
-                    for (int q = 1; q < R; ++q) {
-                        Cx &x = v[reg<s, true>(i, q)];
-                        x = cmul(x, w);
-                        if (q < R - 1) w = cmul(w, w1);
-                    }
+                if constexpr (by_powers<s>()) {
+                    powers<s>(tw, j, [&](int q, Cx w) { v[reg<s, true>(i, q)] = cmul(v[reg<s, true>(i, q)], w); });
                 } else {
 #pragma unroll
                     for (int q = 1; q < R; ++q) {
@@ -456,15 +470,8 @@ struct Block : Radix<LOG_L, E_, direct_max_ls(2 * sizeof(Real), LOG_L, digit_bit
         for (int i = 0; i < E / R; ++i) {
             if constexpr (s < NS - 1) {
                 const int j = Rx::beta(s, tp, i) & ((1 << LSS) - 1);
-                if constexpr (running<s>()) {
-                    const Cx w1 = twid<s>(tw, j, 1);
-                    Cx w = w1;
-#pragma unroll
-                    for (int q = 1; q < R; ++q) {
-                        Cx &x = v[reg<s, true>(i, q)];
-                        x = cmulc(x, w);
-                        if (q < R - 1) w = cmul(w, w1);
-                    }
+                if constexpr (by_powers<s>()) {
+                    powers<s>(tw, j, [&](int q, Cx w) { v[reg<s, true>(i, q)] = cmulc(v[reg<s, true>(i, q)], w); });
                 } else {
 #pragma unroll
                     for (int q = 1; q < R; ++q) {
