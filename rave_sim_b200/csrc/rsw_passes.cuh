@@ -456,11 +456,6 @@ template <int LOG_L2, int E> struct RowTab {
     static constexpr int RO = SHORT ? 0 : 64 + NQ;  // first register part of the chirp factors
     static constexpr int NCH = RO + E;
 };
-// entries of the row kernel's chirp table (chirp_table_kernel)
-template <typename Real, int LOG_L2, int E> struct ChirpTab {
-    static constexpr bool PRODUCT = sizeof(Real) == 8 && RowTab<LOG_L2, E>::SHORT;
-    static constexpr int ENTRIES = PRODUCT ? (1 + ilog2(E)) * ((1 << LOG_L2) / E) : 1 << LOG_L2;
-};
 // Threads of the row kernel. Single rows of at most 2^11 samples evaluate the
 // transfer function per sample in FP64: 256 threads fill a table of it in
 // shared memory before the kernel waits for the one before it, then all but
@@ -585,9 +580,7 @@ __global__ void __launch_bounds__(row_threads<LOG_L2, Block<Real, LOG_L2, 1, E>:
                 } else {
                     const int fo = B::freq_off(idx - RO);
                     const int64_t sr = (fo & (L >> 1)) ? int64_t(fo) - L : int64_t(fo);
-                    double t = frac_dd(g1h, g1l, double(kbase * sr));
-                    if constexpr (ChirpTab<Real, LOG_L2, E>::PRODUCT) t += frac_dd(m * m * g_hi, m * m * g_lo, double(sr * sr));
-                    w = cis_turns(t);
+                    w = cis_turns(frac_dd(g1h, g1l, double(kbase * sr)));
                 }
                 if constexpr (B::LIFT) {
                     if (idx < RO) reinterpret_cast<double2 *>(chp)[idx] = w;
@@ -621,7 +614,7 @@ __global__ void __launch_bounds__(row_threads<LOG_L2, Block<Real, LOG_L2, 1, E>:
                 // wrote it: a column pass, which waited for it, lies between)
                 if (a.pr.has_h) {
                     const char *h3 = static_cast<const char *>(BATCH ? a.bpr[row >> log_m].h3 : a.pr.h3);
-                    for (int k = tp; k < ChirpTab<Real, LOG_L2, E>::ENTRIES / 8; k += B::NT)
+                    for (int k = tp; k < L / 8; k += B::NT)
                         asm volatile("prefetch.global.L1 [%0];" ::"l"(h3 + k * 128));
                 }
             }
@@ -649,6 +642,19 @@ __global__ void __launch_bounds__(row_threads<LOG_L2, Block<Real, LOG_L2, 1, E>:
             }
         };
         Cx v[E];
+        // complex128 rows of few warps: the chirp table's entries in flight with
+        // the samples, all at once (loaded where they are used, four at a time,
+        // they wait for L2 one batch after the other: the split steps of a
+        // simulation at 2^16 450 against 437 us)
+        constexpr bool EARLY = SHORT && CHIRP && !TABLE && !B::LIFT;
+        [[maybe_unused]] Cx h[EARLY ? E : 1];
+        if constexpr (EARLY) {
+            if (a.pr.has_h) {
+                const Cx *h3 = static_cast<const Cx *>(BATCH ? a.bpr[row >> log_m].h3 : a.pr.h3) + tp;
+#pragma unroll
+                for (int r = 0; r < E; ++r) h[r] = __ldg(h3 + r * B::T);
+            }
+        }
         if (!(flags & PF_SPEC_IN)) {
 #pragma unroll
             for (int r = 0; r < E; ++r) v[r] = (flags & PF_ONES) ? one_c<Cx>() : __ldcg(gin + B::first_pos(tp, r));
@@ -729,40 +735,12 @@ __global__ void __launch_bounds__(row_threads<LOG_L2, Block<Real, LOG_L2, 1, E>:
                     };
                     if (cut_span == 0) rotate(std::false_type{});
                     else rotate(std::true_type{});
-                } else if constexpr (ChirpTab<Real, LOG_L2, E>::PRODUCT) {
-                // complex128: with f = fbase, G3 = G M^2 the quadratic part is
-                // exp(2 pi i G3 (f^2 + s_r^2 + 2 f s_r)). s_r is a sum over the bits of r,
-                // so the cross term is a product of LE factors X[b] per thread: 1 +
-                // LE table entries a thread in place of E; exp(2 pi i G3 s_r^2) is folded
-                // into R[r]. The same number of products, and the loads are one
-                // short batch instead of E / 4 that wait for L2 one after the
-                // other: a run of short split steps at 2^16 325 -> 308 us. Longer
-                // rows hide that wait behind their other warps and gained nothing
-                // (2^22 23.5 against 23.6 ps per sample), so they keep the table.
-                constexpr int LE = ilog2(E);
-                const double2 *xt = reinterpret_cast<const double2 *>(h3) + tp;
-                double2 X[LE];
-#pragma unroll
-                for (int b = 0; b < LE; ++b) X[b] = __ldg(xt + (b + 1) * B::T);
-                double2 hi[E / 4], lo[4];
-                hi[0] = cmul(thread_chirp, __ldg(xt));
-#pragma unroll
-                for (int b = 2; b < LE; ++b)
-#pragma unroll
-                    for (int k = 0; k < (1 << (b - 2)); ++k) hi[k + (1 << (b - 2))] = cmul(hi[k], X[b]);
-                lo[1] = X[0];
-                lo[2] = X[1];
-                lo[3] = cmul(X[0], X[1]);
+                } else if constexpr (SHORT) {
                 const auto multiply = [&](auto cut) {
 #pragma unroll
                     for (int r = 0; r < E; ++r) {
-                        double2 h = hi[r >> 2];
-                        if (r & 3) h = cmul(h, lo[r & 3]);
-                        v[r] = cmul(v[r], cmul(h, chp[RO + r]));
-                        if constexpr (decltype(cut)::value) v[r] = zero_cut(r, v[r]);
-                        // a compiler-only barrier per 4 samples keeps the R[r] loads
-                        // from being issued all ahead and held live
-                        if (r % 4 == 3) asm volatile("" ::: "memory");
+                        const Cx x = cmul(v[r], cmul(cmul(thread_chirp, chp[RO + r]), h[r]));
+                        v[r] = decltype(cut)::value ? zero_cut(r, x) : x;
                     }
                 };
                 if (cut_span == 0) multiply(std::false_type{});
@@ -1125,34 +1103,23 @@ __global__ void __launch_bounds__(Block<Real, LOG_L1, C, E>::NT,
     col_pass<Real, LOG_L1, C, E, DET, BATCH>(a);
 }
 
-// The row kernel's chirp table, G3 = G M^2 (16-byte entries):
-// exp(2 pi i G3 k2s^2) for every register r of thread tp at r * T + tp ({cos, sin}
-// for complex128, the lifting form for complex64). Short complex128 rows
-// (PRODUCT): exp(2 pi i G3 f^2) of the thread's frequency part f at tp, and
-// exp(2 pi i 2 G3 f s) at (b + 1) * T + tp for the register part s of r = 2^b
-// (negative for the top frequency bit).
+// The row kernel's chirp table, G3 = G M^2 (16-byte entries): exp(2 pi i G3
+// k2s^2) for every register r of thread tp at r * T + tp ({cos, sin} for
+// complex128, the lifting form for complex64).
 template <typename Real, int LOG_L2, int E>
 __global__ void chirp_table_kernel(typename LiftT<Real>::T *__restrict__ out, double g3_hi, double g3_lo) {
     using B = Block<Real, LOG_L2, 1, E>;
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     pass_wait();  // the table's last reader
     pass_release();
-    if (idx >= ChirpTab<Real, LOG_L2, E>::ENTRIES) return;
+    if (idx >= B::L) return;
     const int r = idx / B::T, tp = idx % B::T;
-    if constexpr (!ChirpTab<Real, LOG_L2, E>::PRODUCT) {
-        const int half2 = 1 << (LOG_L2 - 1);
-        const int k2 = B::last_freq(tp, r);
-        const double k2s = double(k2 >= half2 ? k2 - 2 * half2 : k2);
-        const double2 w = cis_turns(frac_dd(g3_hi, g3_lo, k2s * k2s));
-        if constexpr (sizeof(Real) == 4) out[idx] = lift_of(w);
-        else out[idx] = w;
-    } else {
-        const int64_t f = B::freq_base(tp);
-        const int fo = r > 0 ? B::freq_off(1 << (r - 1)) : 0;
-        const int64_t s = (fo & (B::L >> 1)) ? int64_t(fo) - B::L : int64_t(fo);
-        out[idx] = cis_turns(r > 0 ? frac_dd(2.0 * g3_hi, 2.0 * g3_lo, double(f * s))
-                                   : frac_dd(g3_hi, g3_lo, double(f * f)));
-    }
+    const int half2 = 1 << (LOG_L2 - 1);
+    const int k2 = B::last_freq(tp, r);
+    const double k2s = double(k2 >= half2 ? k2 - 2 * half2 : k2);
+    const double2 w = cis_turns(frac_dd(g3_hi, g3_lo, k2s * k2s));
+    if constexpr (sizeof(Real) == 4) out[idx] = lift_of(w);
+    else out[idx] = w;
 }
 
 void count_launch();
@@ -1335,8 +1302,7 @@ static cudaError_t col_impl(const PassArgs &a, cudaStream_t s) {
 }
 
 template <typename Real, int LG, int E> static cudaError_t chirp_impl(void *out, double hi, double lo, cudaStream_t s) {
-    return launch_dependent(chirp_table_kernel<Real, LG, E>,
-                            (ChirpTab<Real, LG, E>::ENTRIES + 255) / 256, 256, 0, s, false,
+    return launch_dependent(chirp_table_kernel<Real, LG, E>, ((1 << LG) + 255) / 256, 256, 0, s, false,
                             static_cast<typename LiftT<Real>::T *>(out), hi, lo);
 }
 }  // namespace rsw
