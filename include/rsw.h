@@ -93,7 +93,11 @@ typedef struct {
     int row_e, col_e, mid_e;
 } rsw_tuning;
 rsw_status rsw_plan_create_tuned(rsw_plan *out, int64_t n, int dtype, const rsw_tuning *tuning);
-/* The plan's effective choices (of its length-M plan for Bluestein lengths). */
+/* The plan's effective choices (of its length-M plan for Bluestein lengths).
+ * Short fields that run two levels by default (complex128 2^12 and 2^13,
+ * complex64 to 2^14) report levels = 0: they evaluate the transfer function
+ * per sample with the reference's roundings, as one row does, where a split
+ * that a tuning names evaluates the phase exactly. */
 rsw_status rsw_plan_tuning(rsw_plan plan, rsw_tuning *tuning);
 /* Register the tuning that later rsw_plan_create / rsw_sim_create calls use
  * for this n and dtype (process-wide; tuning == NULL removes it). The

@@ -49,6 +49,7 @@ cudaError_t launch_detect(const void *u, const int64_t *bounds, const double *co
 cudaError_t launch_zero(double *p, int64_t n, cudaStream_t s);
 cudaError_t launch_fill_ones(void *u, int64_t n, bool dbl, cudaStream_t s);
 cudaError_t launch_chirp_table(void *out, int log_n2, double hi, double lo, bool dbl, int e, cudaStream_t s);
+cudaError_t launch_transfer_table(double2 *out, int64_t n, const SpecLevels &v, const PropArgs &p, cudaStream_t s);
 cudaError_t launch_blue_pre(const void *in, void *w, int64_t n, int64_t m, const double2 *b, bool conj_in, bool dbl,
                             cudaStream_t s);
 cudaError_t launch_blue_mul(void *w, const double2 *bh, int64_t m, bool dbl, cudaStream_t s);
@@ -315,6 +316,7 @@ static constexpr int ROW_MAX_C128 = 13, COL_MAX_C128 = 11;
 // and for tunings
 static constexpr int COL_TUNE_MAX_C128 = 12;
 static constexpr int ROW_MAX_C64 = 14, COL_MAX_C64 = 12;
+static constexpr int SINGLE_ROW_MAX = 11;  // longest field that takes one row by default
 static std::atomic<uint64_t> g_api_calls{0};
 
 struct rsw_plan_s {
@@ -326,6 +328,13 @@ struct rsw_plan_s {
     int device = 0;
     int row_e = 16, col_e = 16, mid_e = 16;  // elements per thread of the row / column / middle kernels
     int prop_mode = RSW_PROP_FRESNEL;        // transfer function of propagate and of simulations
+    // Two levels by default although one row could hold the field: the transfer
+    // function is evaluated per sample as there, with the reference's own
+    // roundings of the phase (the chirp form evaluates it exactly, which differs
+    // from the reference by up to 1e-10). propagate does so in the row pass and
+    // keeps no table in the plan, so that calls on several streams or under
+    // capture share it freely; simulations keep whole functions (table_for).
+    bool per_sample = false;
     DevBuf tw_row, tw_col, tw_mid, tw4_lo, tw4_hi, tw4b_lo, tw4b_hi;
     // Rows whose default is not 16 samples per thread: the count and the table
     // of the other propagator (the exact one has kernels of 16 only), exchanged
@@ -483,7 +492,9 @@ static rsw_status tuned_split(int lg, int dtype, const rsw_tuning &t, int *l1, i
     return RSW_OK;
 }
 
-static rsw_status plan_split(int64_t n, int dtype, int *log_n, int *l1, int *lb, int *lr, const rsw_tuning *t) {
+// dflt: the split is the default one, neither a tuning's nor the environment's.
+static rsw_status plan_split(int64_t n, int dtype, int *log_n, int *l1, int *lb, int *lr, const rsw_tuning *t,
+                             bool *dflt) {
     if (n < 16 || (n & (n - 1)) != 0)
         return fail(RSW_ERR_UNSUPPORTED, "N = %lld: this version supports powers of two >= 16", (long long)n);
     int lg = 0;
@@ -492,6 +503,7 @@ static rsw_status plan_split(int64_t n, int dtype, int *log_n, int *l1, int *lb,
     const int col_max = dtype == RSW_C128 ? COL_MAX_C128 : COL_MAX_C64;
     *log_n = lg;
     *lb = 0;
+    *dflt = false;
     if (t && t->levels != 0) return tuned_split(lg, dtype, *t, l1, lb, lr);
     // RSW_SPLIT3 = "l1,lb,lr" forces a three-level split (tests and tuning sweeps)
     const char *ov3 = std::getenv("RSW_SPLIT3");
@@ -516,12 +528,13 @@ static rsw_status plan_split(int64_t n, int dtype, int *log_n, int *l1, int *lb,
             return RSW_OK;
         }
     }
+    *dflt = true;
     // Single rows up to 2^11 samples only: one CTA runs the whole transform,
     // with the transfer function evaluated per sample. A propagation of 2^13
-    // complex128 samples takes 31 us on one row and 16 us as short passes, of
-    // 2^14 complex64 35 and 16 us, a forward FFT 19 and 13 us (2^14 complex64
+    // complex128 samples takes 31 us on one row and 12 us as short passes, of
+    // 2^14 complex64 35 and 11 us, a forward FFT 19 and 13 us (2^14 complex64
     // 25 and 13). At 2^11 both are equal, and the FFT is 1 us faster on one row.
-    if (lg <= 11) {
+    if (lg <= SINGLE_ROW_MAX) {
         *l1 = 0;
         *lr = lg;
         return RSW_OK;
@@ -811,7 +824,7 @@ static rsw_status run_mid(const rsw_plan_s *p, const PassArgs &base, bool forwar
 // samples) and switch `pr` to the chirp form. Multi-level plans only: the
 // spectrum index of a row sample is kbase + M k2 with M = N1 Nb.
 static rsw_status prepare_chirp(const rsw_plan_s *p, PropArgs &pr, void *table, cudaStream_t s) {
-    if (p->log_n1 == 0 || !pr.has_h || pr.exact) return RSW_OK;
+    if (p->log_n1 == 0 || p->per_sample || !pr.has_h || pr.exact) return RSW_OK;
     double g_hi, g_lo;
     chirp_constant(pr, p->n, &g_hi, &g_lo);
     const double msq = std::ldexp(1.0, 2 * (p->log_n1 + p->log_nb));  // exact power of two
@@ -893,7 +906,8 @@ static rsw_status create_plan(rsw_plan *out, int64_t n, int dtype, const rsw_tun
     // lengths that are not a power of two, and powers of two below 16
     if (n >= 1 && ((n & (n - 1)) != 0 || n < 16)) return create_blue_plan(out, n, dtype);
     int lg = 0, l1 = 0, lb = 0, lr = 0;
-    CHECK(plan_split(n, dtype, &lg, &l1, &lb, &lr, t));
+    bool dflt = false;
+    CHECK(plan_split(n, dtype, &lg, &l1, &lb, &lr, t, &dflt));
     std::unique_ptr<rsw_plan_s> p(new (std::nothrow) rsw_plan_s());
     if (!p) return fail(RSW_ERR_NOMEM, "host allocation failed");
     p->n = n;
@@ -903,6 +917,7 @@ static rsw_status create_plan(rsw_plan *out, int64_t n, int dtype, const rsw_tun
     p->log_nb = lb;
     p->log_nr = lr;
     p->log_n2 = lb + lr;
+    p->per_sample = dflt && l1 > 0 && lg <= (dtype == RSW_C128 ? ROW_MAX_C128 : ROW_MAX_C64);
     CU(cudaGetDevice(&p->device));
     CHECK(choose_tuning(p.get(), t));
     CHECK(p->dbl() ? plan_tables<double>(p.get()) : plan_tables<float>(p.get()));
@@ -1051,8 +1066,10 @@ rsw_status rsw_plan_create_tuned(rsw_plan *out, int64_t n, int dtype, const rsw_
 rsw_status rsw_plan_tuning(rsw_plan p, rsw_tuning *t) {
     if (!p || !t) return fail(RSW_ERR_INVALID, "NULL argument");
     if (p->blue) return rsw_plan_tuning(p->inner.get(), t);  // the transforms of length m do the work
-    t->levels = p->log_n1 == 0 ? 1 : p->three() ? 3 : 2;
-    t->log_rows = p->log_n1;
+    // a plan that evaluates the transfer function per sample is the default
+    // split's only (levels = 0: the split follows from the length)
+    t->levels = p->per_sample ? 0 : p->log_n1 == 0 ? 1 : p->three() ? 3 : 2;
+    t->log_rows = p->per_sample ? 0 : p->log_n1;
     t->log_mid = p->log_nb;
     t->row_e = p->row_e;
     t->col_e = p->log_n1 > 0 ? p->col_e : 0;
@@ -1094,6 +1111,7 @@ rsw_status rsw_autotune_batch(int64_t n, int dtype, int64_t fields, int reps, rs
     const int col_max = dtype == RSW_C128 ? COL_MAX_C128 : COL_MAX_C64;
     std::vector<rsw_tuning> cands;
     if (lg <= row_max) cands.push_back(rsw_tuning{1, 0, 0, 16, 0, 0});
+    if (lg <= row_max && lg > SINGLE_ROW_MAX && !env_overrides()) cands.push_back(rsw_tuning{0, 0, 0, 16, 16, 0});
     const bool c128 = dtype == RSW_C128;
     const int col_tune = c128 ? COL_TUNE_MAX_C128 : col_max;
     if (lg <= row_max + col_tune) {
@@ -1423,7 +1441,7 @@ rsw_status rsw_propagate(rsw_plan p, void *u, void *U, double dx, double wl, dou
     a.pr = make_prop(p->n, dx, wl, dz, cutoff_freq, dz != 0.0, p->prop_mode == RSW_PROP_EXACT);
     if (p->blue) return blue_propagate(p, u, U, a.pr, skip_fft != 0, s);
     const bool two = p->log_n1 > 0;
-    if (two && a.pr.has_h && !a.pr.exact) {
+    if (two && !p->per_sample && a.pr.has_h && !a.pr.exact) {
         CHECK(p->h3_call.alloc(size_t(int64_t(1) << p->log_nr) * 16));  // 16-byte entries
         CHECK(prepare_chirp(p, a.pr, p->h3_call.p, s));
     }
@@ -1747,6 +1765,7 @@ struct rsw_sim_s {
     DevBuf buf[2];
     DevBuf mat_db, mat_fac;  // per-run sample material tables
     std::vector<std::unique_ptr<DevBuf>> h3_pool;  // chirp tables, one per distinct dz of a run
+    std::vector<std::unique_ptr<DevBuf>> h_pool;   // short plans: whole transfer functions (Runner::table_for)
     int last_field = -1;
     TimingLog tl;
     int64_t split_steps = 0;
@@ -1805,6 +1824,7 @@ struct Runner {
     // per-run material factors: per element [fa? ...]
     std::vector<std::vector<cplx>> db;  // deltabeta per element (gratings: a,b,sub; samples: materials 1..)
     std::vector<double> chirp_dz;       // dz of each built chirp table of this run (slot = index)
+    std::vector<std::pair<double, double>> table_keys;  // (dz, cutoff angle) of each whole transfer function
     // Lockstep batches (rsw_sim_run_batch): nb instances of the same field
     // length in consecutive N-sample slices of the batch buffers; instance 0's
     // values stand in the common arguments, the wavelength-dependent ones of
@@ -1821,7 +1841,7 @@ struct Runner {
 
     // chirp table for a distance dz at this run's wavelength (built on first use)
     rsw_status chirp_for(PropArgs &pr, double dz) {
-        if (P->log_n1 == 0 || !pr.has_h || pr.exact) return RSW_OK;
+        if (P->log_n1 == 0 || P->per_sample || !pr.has_h || pr.exact) return RSW_OK;
         size_t slot = 0;
         while (slot < chirp_dz.size() && chirp_dz[slot] != dz) ++slot;
         const bool fresh = slot == chirp_dz.size();
@@ -1838,6 +1858,29 @@ struct Runner {
         pr.g_hi = g_hi;
         pr.g_lo = g_lo;
         pr.h3 = S->h3_pool[slot]->p;
+        return RSW_OK;
+    }
+
+    // Short plans (rsw_plan_s::per_sample): the whole transfer function of every
+    // instance over dz with cutoff ci, N FP64 values in the spectrum layout
+    // (at most 256 KB), evaluated once per run in place of once per split step
+    rsw_status table_for(PropArgs &pr, double dz, int ci) {
+        const std::pair<double, double> key(dz, S->cutoff_angles[size_t(ci)]);
+        const size_t slot = size_t(std::find(table_keys.begin(), table_keys.end(), key) - table_keys.begin());
+        if (slot == table_keys.size()) {
+            table_keys.push_back(key);
+            if (S->h_pool.size() <= slot) S->h_pool.emplace_back(new DevBuf());
+            CHECK(S->h_pool[slot]->alloc(size_t(P->n) * size_t(nb) * sizeof(double2)));
+            for (int b = 0; b < nb; ++b) {
+                const PropArgs q = make_prop(P->n, S->d.dx, wls[size_t(b)], dz,
+                                             nb > 1 ? cuts[size_t(b)][size_t(ci)] : cut[size_t(ci)], true);
+                cudaError_t e = launch_transfer_table(static_cast<double2 *>(S->h_pool[slot]->p) + int64_t(b) * P->n,
+                                                      P->n, spec_levels(P), q, st);
+                if (e != cudaSuccess) return fail(RSW_ERR_CUDA, "transfer function: %s", cudaGetErrorString(e));
+            }
+        }
+        pr = PropArgs{};
+        pr.table = static_cast<const double2 *>(S->h_pool[slot]->p);
         return RSW_OK;
     }
 
@@ -1910,8 +1953,11 @@ struct Runner {
         a.pr = make_prop(P->n, S->d.dx, wl, dz, cut[size_t(ci)], dz != 0.0, P->prop_mode == RSW_PROP_EXACT);
         if (nb > 1) {
             a.n = P->n * nb;
-            CHECK(batch_prop(a.pr, dz, ci, &a.bpr));
+            if (P->per_sample && a.pr.has_h) CHECK(table_for(a.pr, dz, ci));
+            else CHECK(batch_prop(a.pr, dz, ci, &a.bpr));
             a.btr = tr.kind != TR_NONE ? btr : nullptr;
+        } else if (P->per_sample && a.pr.has_h && !a.pr.exact) {
+            CHECK(table_for(a.pr, dz, ci));
         } else {
             CHECK(chirp_for(a.pr, dz));
         }
@@ -2747,9 +2793,9 @@ rsw_status rsw_sim_run_batch(rsw_sim S, const rsw_source *srcs, int64_t n_source
         if (!(runs[b].energy_ev > 0) && !(runs[b].wavelength_m > 0))
             return fail(RSW_ERR_INVALID, "source %lld: energy or wavelength must be positive", (long long)b);
     const rsw_plan_s *P = S->plan;
-    // lockstep needs the two- or three-level passes with the chirp form of the
-    // Fresnel kernel and the fused detection; everything else runs the
-    // sources one after the other, with the same results
+    // lockstep needs the two- or three-level passes with the Fresnel kernel
+    // and the fused detection; everything else runs the sources one after the
+    // other, with the same results
     const bool lockstep = count > 1 && P->log_n1 > 0 && !P->blue && P->prop_mode == RSW_PROP_FRESNEL &&
                           S->hist_dz == 0.0 && S->keypoints.empty() && S->final_fields.empty() &&
                           !S->els.empty() && S->geom.n_pix > 0 && same_kind;

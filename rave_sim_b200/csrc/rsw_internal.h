@@ -61,8 +61,9 @@ struct PropArgs {
     // per sample (no chirp form); evanescent fx^2 >= inv_wl2 is zeroed.
     int exact;
     double inv_wl, inv_wl2, z2pi;
-    // Convolution plans (lengths that are not a power of two): the spectrum is
-    // multiplied by this FP64 table instead, in the spectrum layout (SpecLevels)
+    // Convolution plans (lengths that are not a power of two) and simulations on
+    // short two-level plans: the spectrum is multiplied by this FP64 table
+    // instead, in the spectrum layout (SpecLevels)
     const double2 *table;
 };
 

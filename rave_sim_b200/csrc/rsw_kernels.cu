@@ -118,6 +118,16 @@ __device__ __forceinline__ int64_t spec_addr(int64_t k, const SpecLevels &v) {
     const int64_t row = (int64_t(digitpos_i(k1, v.log_n1, v.rb_n1)) << v.log_nb) + digitpos_i(kb, v.log_nb, v.rb_nb);
     return seq + (row << v.log_nr) + row_place(kr, v);
 }
+// The transfer function (with its cutoff) of a whole field in the spectrum
+// layout, for row passes that multiply by a table: evaluated per sample in
+// FP64 with the reference's roundings. A few 10^4 samples, latency-bound.
+__global__ void transfer_table_kernel(double2 *__restrict__ out, int64_t n, SpecLevels v, PropArgs p) {
+    pass_wait();  // the table's last reader
+    pass_release();
+    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+    for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < n; k += stride)
+        out[spec_addr(k, v)] = prop_apply(p, k, k >= n / 2 ? k - n : k, make_double2(1.0, 0.0));
+}
 template <typename Cx>
 __global__ void spec_to_natural_kernel(const Cx *__restrict__ in, Cx *__restrict__ out, int64_t n, SpecLevels v) {
     pass_wait();
@@ -334,6 +344,9 @@ cudaError_t launch_natural_to_spec(const void *in, void *out, int64_t n, const S
                                    cudaStream_t s) {
     if (dbl) return spec_permute<double2, false>((const double2 *)in, (double2 *)out, n, v, s);
     return spec_permute<float2, false>((const float2 *)in, (float2 *)out, n, v, s);
+}
+cudaError_t launch_transfer_table(double2 *out, int64_t n, const SpecLevels &v, const PropArgs &p, cudaStream_t s) {
+    return launch_dependent(transfer_table_kernel, grid_for(n, 64), 64, 0, s, false, out, n, v, p);
 }
 cudaError_t launch_trans(void *u, int64_t n, const TransArgs &tr, bool dbl, cudaStream_t s) {
     ++g_launches;

@@ -456,11 +456,15 @@ template <int LOG_L2, int E> struct RowTab {
     static constexpr int RO = SHORT ? 0 : 64 + NQ;  // first register part of the chirp factors
     static constexpr int NCH = RO + E;
 };
-// Threads of the row kernel. Single rows of at most 2^11 samples evaluate the
-// transfer function per sample in FP64: 256 threads fill a table of it in
-// shared memory before the kernel waits for the one before it, then all but
-// the row's own leave (launched so only where the table is used).
-template <int LOG_L2, int NT, bool CHIRP> constexpr int row_threads() { return !CHIRP && LOG_L2 <= 11 ? 256 : NT; }
+// Threads of the row kernel. Rows of at most 2^11 samples that evaluate the
+// transfer function per sample in FP64: in launches of few rows a CTA has up to
+// 256 threads that fill a table of its row's function in shared memory before
+// the kernel waits for the one before it, then all but the row's own leave
+// (row_launch: such a launch has one row per CTA, or single rows, which are
+// transforms of their own with the same function).
+template <int LOG_L2, int NT, bool CHIRP> constexpr int row_threads() {
+    return CHIRP || LOG_L2 > 11 ? NT : LOG_L2 >= 8 ? 256 : LOG_L2 >= 5 ? 1 << LOG_L2 : 32;
+}
 
 // TABLE: the spectrum is multiplied by a table (PropArgs::table) in place of a
 // transfer function (with CHIRP set: no per-sample phases). Its own kernel, so
@@ -485,22 +489,35 @@ __global__ void __launch_bounds__(row_threads<LOG_L2, Block<Real, LOG_L2, 1, E>:
     const int tp = threadIdx.x;
     const int flags = a.flags;
     const int64_t rows = a.n >> LOG_L2;
+    const int log_m = a.log_n1 + a.log_nb;  // spectrum index k = kbase + 2^log_m * k2
+    // row -> (p1, pb): spectrum index base kbase = k1 + N1 kb (rows beyond one
+    // transform belong to the next one of a batch)
+    const auto row_k1 = [&](int64_t row) {
+        return digitrev_w((row >> a.log_nb) & ((int64_t(1) << a.log_n1) - 1), a.log_n1, a.rb_n1);
+    };
+    const auto row_kb = [&](int64_t row) { return digitrev_w(row & ((int64_t(1) << a.log_nb) - 1), a.log_nb, a.rb_nb); };
+    const auto row_k = [&](int64_t row) { return row_k1(row) + (row_kb(row) << a.log_n1); };
     constexpr int HT = row_threads<LOG_L2, B::NT, CHIRP>();
     if (HT == B::NT || tp < B::NT) B::load_twiddles(tw, static_cast<const Tw *>(a.tw_row));
-    // the transfer function of a single row, register r of thread t at r * T + t;
-    // (0, 0) marks a zeroed component (the others have modulus 1)
-    double2 *const hs = reinterpret_cast<double2 *>(tabs);
+    // the transfer function of the CTA's row (row_threads), register r of thread
+    // t at r * T + t (complex64: in lifting form); zeros mark a zeroed component
+    // (the others have modulus 1, and their lifting forms the sign 1 or -1)
+    Lf *const hs = tabs + 2 * (NV + NCH);
     bool h_table = false;
     if constexpr (HT > B::NT) {
         h_table = blockDim.x > B::NT;
         if (h_table) {
+            const int64_t k0 = row_k(blockIdx.x);
             for (int k = tp; k < L; k += HT) {
-                double2 H = make_double2(0.0, 0.0);
+                Lf H{};
                 double s, c, ph;
-                if (!(a.pr.has_cut && k >= a.pr.cut_lo && k < a.pr.cut_hi) &&
-                    prop_phase_any(a.pr, k >= L / 2 ? int64_t(k) - L : int64_t(k), &ph)) {
+                const int64_t kn = k0 + (int64_t(k) << log_m);
+                const int64_t ks = k0 + int64_t(k >= L / 2 ? k - L : k) * (int64_t(1) << log_m);
+                if (!(a.pr.has_cut && kn >= a.pr.cut_lo && kn < a.pr.cut_hi) && prop_phase_any(a.pr, ks, &ph)) {
                     sincos_phase(ph, &s, &c);
-                    H = make_double2(a.pr.A.x * c - a.pr.A.y * s, a.pr.A.x * s + a.pr.A.y * c);
+                    const double2 h = make_double2(a.pr.A.x * c - a.pr.A.y * s, a.pr.A.x * s + a.pr.A.y * c);
+                    if constexpr (B::LIFT) H = lift_of(h);
+                    else H = h;
                 }
                 const int p = int(digitpos_rt(k, LOG_L2, B::RB)), o = p % E;
                 const int r = o / B::RL * B::RL + brev_bits(o % B::RL, ilog2(B::RL));
@@ -512,7 +529,6 @@ __global__ void __launch_bounds__(row_threads<LOG_L2, Block<Real, LOG_L2, 1, E>:
     }
     const int64_t nmask = (int64_t(1) << a.tw_log) - 1;
     const double tw_scale = a.tw_scale;
-    const int log_m = a.log_n1 + a.log_nb;  // spectrum index k = kbase + 2^log_m * k2
     // A forward + inverse row starts and ends with the stage-0 positions of
     // each thread, so the next row may overwrite the data buffer without a
     // barrier; every other flow ends its row with one.
@@ -543,11 +559,8 @@ __global__ void __launch_bounds__(row_threads<LOG_L2, Block<Real, LOG_L2, 1, E>:
         Lf *chp = vec + NV;
         [[maybe_unused]] double2 thread_chirp = make_double2(1.0, 0.0);  // SHORT: this thread's P Q
         [[maybe_unused]] Lf thread_tw{};                                 // SHORT: its four-step factor
-        // row -> (p1, pb): spectrum index base kbase = k1 + N1 kb; the
-        // conjugate four-step twiddle of the innermost split uses tw_k
-        // (rows beyond one transform belong to the next one of a batch)
-        const int64_t k1 = digitrev_w((row >> a.log_nb) & ((int64_t(1) << a.log_n1) - 1), a.log_n1, a.rb_n1);
-        const int64_t kb = digitrev_w(row & ((int64_t(1) << a.log_nb) - 1), a.log_nb, a.rb_nb);
+        // the conjugate four-step twiddle of the innermost split uses tw_k
+        const int64_t k1 = row_k1(row), kb = row_kb(row);
         const int64_t kbase = k1 + (kb << a.log_n1);
         const int64_t tw_k = a.log_nb > 0 ? kb : k1;
         if (CHIRP && !TABLE && a.pr.has_h) {
@@ -771,10 +784,9 @@ __global__ void __launch_bounds__(row_threads<LOG_L2, Block<Real, LOG_L2, 1, E>:
         } else if (h_table) {
 #pragma unroll
             for (int r = 0; r < E; ++r) {
-                const double2 H = hs[r * B::T + tp];
-                const bool zero = H.x == 0.0 && H.y == 0.0;
-                if constexpr (B::LIFT) v[r] = zero ? Cx{} : rot(v[r], lift_of(H));
-                else v[r] = zero ? Cx{} : cmul(v[r], H);
+                const Lf H = hs[r * B::T + tp];
+                if constexpr (B::LIFT) v[r] = H.z == 0.f ? Cx{} : rot(v[r], H);
+                else v[r] = H.x == 0.0 && H.y == 0.0 ? Cx{} : cmul(v[r], H);
             }
         } else if (a.pr.has_h || a.pr.has_cut) {
             const int64_t half2 = int64_t(1) << (LOG_L2 - 1);
@@ -1140,15 +1152,16 @@ template <typename K> static int64_t resident_ctas(K kernel, int threads, size_t
 // Launch set-up of one kernel, per device: the dynamic shared-memory limit is
 // a per-device attribute of the kernel and the resident CTA count depends on
 // the device, so both are taken once for each device the kernel launches on
-// (the device current at the launch). cap[1] is the CTA count at the
-// second shared-memory size (the column kernel without its factor tables).
+// (the device current at the launch). cap[1] is the CTA count at the second
+// thread count and shared-memory size (the column kernel without its factor
+// tables, the row kernel with its transfer function's).
 constexpr int LAUNCH_MAX_DEVICES = 64;
 struct LaunchSetup {
     cudaError_t attr = cudaSuccess;
     int64_t cap[2] = {1, 1};
 };
 template <typename K>
-static const LaunchSetup *launch_setup(K kernel, int threads, size_t smem, size_t smem2, LaunchSetup *table,
+static const LaunchSetup *launch_setup(K kernel, int threads, size_t smem, int threads2, size_t smem2, LaunchSetup *table,
                                        std::once_flag *once) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= LAUNCH_MAX_DEVICES) return nullptr;
@@ -1157,7 +1170,7 @@ static const LaunchSetup *launch_setup(K kernel, int threads, size_t smem, size_
         st.attr = prep(kernel, smem > smem2 ? smem : smem2);
         if (st.attr == cudaSuccess) {
             st.cap[0] = resident_ctas(kernel, threads, smem, dev);
-            st.cap[1] = resident_ctas(kernel, threads, smem2, dev);
+            st.cap[1] = resident_ctas(kernel, threads2, smem2, dev);
         }
     });
     return &table[dev];
@@ -1197,19 +1210,18 @@ template <typename Real, int LG, int E, bool CH, bool TWF, bool BT, bool TABLE =
 static cudaError_t row_launch(const PassArgs &a, cudaStream_t s) {
     using B = Block<Real, LG, 1, E>;
     auto k = row_pass_kernel<Real, LG, E, CH, TWF, BT, TABLE>;
-    const size_t base = (B::SMEM + 15) / 16 * 16;
-    const size_t smem = base + 2 * size_t(RowTab<LG, E>::NV + RowTab<LG, E>::NCH) * 16;
-    // a single row's transfer function in shared memory (row_threads)
+    const size_t smem = (B::SMEM + 15) / 16 * 16 + 2 * size_t(RowTab<LG, E>::NV + RowTab<LG, E>::NCH) * 16;
+    // the row's transfer function in shared memory (row_threads)
     constexpr int HT = row_threads<LG, B::NT, CH>();
-    const bool wide = HT > B::NT && a.log_n1 == 0 && a.pr.has_h;
-    const size_t smem_h = HT > B::NT && base + size_t(B::L) * 16 > smem ? base + size_t(B::L) * 16 : smem;
+    const int64_t rows = a.n >> LG;
+    const size_t smem_h = smem + (HT > B::NT ? size_t(B::L) * 16 : 0);
     static LaunchSetup setup[LAUNCH_MAX_DEVICES];
     static std::once_flag once[LAUNCH_MAX_DEVICES];
-    const LaunchSetup *st = launch_setup(k, B::NT, smem, smem_h, setup, once);
+    const LaunchSetup *st = launch_setup(k, B::NT, smem, HT, smem_h, setup, once);
     if (!st) return cudaErrorInvalidDevice;
     if (st->attr != cudaSuccess) return st->attr;
-    const int64_t cap = st->cap[0];
-    const int64_t rows = a.n >> LG;
+    const bool wide = HT > B::NT && a.pr.has_h && (a.log_n1 == 0 || rows <= st->cap[1]);
+    const int64_t cap = wide ? st->cap[1] : st->cap[0];
     return launch_dependent(k, rows < cap ? rows : cap, wide ? HT : B::NT, wide ? smem_h : smem, s, pass_serial(a, sizeof(typename B::Cx)),
                             a);
 }
@@ -1270,7 +1282,7 @@ static cudaError_t col_launch(const PassArgs &a, cudaStream_t s) {
     const size_t tab = (B::SMEM + 15) / 16 * 16 + ColTab<B::T>::template bytes<C, E, 16>();
     static LaunchSetup setup[LAUNCH_MAX_DEVICES];
     static std::once_flag once[LAUNCH_MAX_DEVICES];
-    const LaunchSetup *st = launch_setup(k, B::NT, tab, plain, setup, once);
+    const LaunchSetup *st = launch_setup(k, B::NT, tab, B::NT, plain, setup, once);
     if (!st) return cudaErrorInvalidDevice;
     if (st->attr != cudaSuccess) return st->attr;
     const bool tables = a.flags & (PF_TW | PF_TWI);

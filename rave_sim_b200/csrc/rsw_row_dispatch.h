@@ -44,10 +44,14 @@ template <typename Real> cudaError_t row_table_dispatch(const PassArgs &a, cudaS
     case L: return chirp ? cudaErrorInvalidValue : RSW_ROW_E(R, L, 16, false);
 
 // multi-level rows take the chirp form of the Fresnel kernel; the exact
-// kernel and single-level rows work per sample.
+// kernel, single-level rows and the rows of short two-level plans (no chirp
+// table) work per sample.
 // BT: the batched kernels (chirp form only; the others return an error)
+static inline bool row_chirp(const PassArgs &a) {
+    return a.log_n1 > 0 && !a.pr.exact && (a.pr.chirp || !a.pr.has_h);
+}
 template <bool BT> cudaError_t row_dispatch_f64(const PassArgs &a, int e, cudaStream_t s) {
-    const bool chirp = a.log_n1 > 0 && !a.pr.exact;
+    const bool chirp = row_chirp(a);
     switch (a.log_n2) {
         RSW_ROW_CASE_S(double, 4) RSW_ROW_CASE_S(double, 5) RSW_ROW_CASE_S(double, 6)
         RSW_ROW_CASE16(double, 7) RSW_ROW_CASE16(double, 8) RSW_ROW_CASE(double, 9)
@@ -56,7 +60,7 @@ template <bool BT> cudaError_t row_dispatch_f64(const PassArgs &a, int e, cudaSt
     }
 }
 template <bool BT> cudaError_t row_dispatch_f32(const PassArgs &a, int e, cudaStream_t s) {
-    const bool chirp = a.log_n1 > 0 && !a.pr.exact;
+    const bool chirp = row_chirp(a);
     switch (a.log_n2) {
         RSW_ROW_CASE_S(float, 4) RSW_ROW_CASE_S(float, 5) RSW_ROW_CASE_S(float, 6) RSW_ROW_CASE16(float, 7)
         RSW_ROW_CASE16(float, 8) RSW_ROW_CASE(float, 9) RSW_ROW_CASE(float, 10) RSW_ROW_CASE8(float, 11)

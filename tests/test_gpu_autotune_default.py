@@ -13,7 +13,7 @@ import rave_sim_b200 as rsw  # noqa: E402
 from rave_sim_b200 import autotune  # noqa: E402
 
 
-@pytest.mark.parametrize("dt,lg", [("c16", 11), ("c16", 16), ("c16", 20), ("c16", 24), ("c16", 26), ("c8", 11),
+@pytest.mark.parametrize("dt,lg", [("c16", 11), ("c16", 13), ("c16", 16), ("c16", 20), ("c16", 24), ("c16", 26), ("c8", 11), ("c8", 14),
                                    ("c8", 16), ("c8", 20), ("c8", 25), ("c8", 26), ("c8", 27)])
 def test_default_is_tried(monkeypatch, dt, lg):
     for v in ("RSW_SPLIT", "RSW_SPLIT3", "RSW_ROW_E", "RSW_COL_E"):
