@@ -879,6 +879,23 @@ static SpecLevels spec_levels(const rsw_plan_s *p) {
                       digit_bits(p->row_e), log_e};
 }
 
+// The forward transform of one field, in -> out (in == out allowed), into the
+// spectrum layout.
+static rsw_status forward_passes(const rsw_plan_s *p, const void *in, void *out, cudaStream_t s) {
+    PassArgs a = base_args(p);
+    a.in = in;
+    a.out = out;
+    if (p->log_n1 > 0) {
+        a.flags = PF_FWD | PF_TW;
+        CHECK(run_col(p, a, s));
+        a.in = out;
+        if (p->three()) CHECK(run_mid(p, a, true, s));
+    }
+    PassArgs r = row_level(p, a);
+    r.flags = PF_FWD | row_tw(p, true, false);
+    return run_row(p, r, s);
+}
+
 // ================================================================== C ABI
 extern "C" {
 
@@ -966,22 +983,31 @@ static rsw_status create_blue_plan(rsw_plan *out, int64_t n, int dtype) {
     }
     CHECK(p->bchirp.upload(b));
     CHECK(p->bhat.upload(bx));
+    // its spectrum, in place: with the inner plan's own level structure the FP64
+    // passes leave it in the inner plan's layout
     rsw_plan p64 = inner;
     std::unique_ptr<rsw_plan_s> own;
     if (dtype != RSW_C128) {
-        CHECK(create_plan(&p64, m, RSW_C128, nullptr));
+        const rsw_tuning same{inner->log_n1 == 0 ? 1 : inner->three() ? 3 : 2, inner->log_n1, inner->log_nb,
+                              inner->row_e, inner->log_n1 > 0 ? inner->col_e : 0, inner->three() ? inner->mid_e : 0};
+        if (create_plan(&p64, m, RSW_C128, &same) != RSW_OK) p64 = nullptr;
         own.reset(p64);
     }
-    CHECK(rsw_fft_forward(p64, p->bhat.p, p->bhat.p, nullptr));
-    CU(cudaDeviceSynchronize());  // done before its plan and scratch go (room for the second copy)
-    own.reset();
-    p->inner->scratch.release();
-    DevBuf nat = std::move(p->bhat);
-    CHECK(p->bhat.alloc(size_t(m) * sizeof(double2)));
-    cudaError_t e = launch_natural_to_spec(nat.p, p->bhat.p, m, spec_levels(p->inner.get()), true, nullptr);
-    if (e != cudaSuccess) return fail(RSW_ERR_CUDA, "bluestein: %s", cudaGetErrorString(e));
-    CU(cudaDeviceSynchronize());
-    nat.release();
+    if (p64) {
+        CHECK(forward_passes(p64, p->bhat.p, p->bhat.p, nullptr));
+        CU(cudaDeviceSynchronize());
+    } else {  // rows of 2^14, which complex128 has not: through natural order
+        CHECK(create_plan(&p64, m, RSW_C128, nullptr));
+        own.reset(p64);
+        CHECK(rsw_fft_forward(p64, p->bhat.p, p->bhat.p, nullptr));
+        CU(cudaDeviceSynchronize());  // done before its plan and scratch go (room for the second copy)
+        own.reset();
+        DevBuf nat = std::move(p->bhat);
+        CHECK(p->bhat.alloc(size_t(m) * sizeof(double2)));
+        cudaError_t e = launch_natural_to_spec(nat.p, p->bhat.p, m, spec_levels(inner), true, nullptr);
+        if (e != cudaSuccess) return fail(RSW_ERR_CUDA, "bluestein: %s", cudaGetErrorString(e));
+        CU(cudaDeviceSynchronize());
+    }
     CHECK(p->bwork.alloc(size_t(m) * p->elem()));
     *out = p.release();
     return RSW_OK;
@@ -1269,16 +1295,7 @@ rsw_status rsw_fft_forward(rsw_plan p, const void *in, void *out, void *stream) 
     if (p->blue) return blue_transform(p, in, out, false, s);
     if (p->log_n1 == 0) return single_fft(p, in, out, p->n, false, s);
     CHECK(need_scratch(p));
-    PassArgs a = base_args(p);
-    a.in = in;
-    a.out = p->scratch.p;
-    a.flags = PF_FWD | PF_TW;
-    CHECK(run_col(p, a, s));
-    a.in = p->scratch.p;
-    if (p->three()) CHECK(run_mid(p, a, true, s));
-    PassArgs r = row_level(p, a);
-    r.flags = PF_FWD | row_tw(p, true, false);
-    CHECK(run_row(p, r, s));
+    CHECK(forward_passes(p, in, p->scratch.p, s));
     cudaError_t e = to_natural(p, p->scratch.p, out, s);
     if (e != cudaSuccess) return fail(RSW_ERR_CUDA, "reorder: %s", cudaGetErrorString(e));
     return RSW_OK;
