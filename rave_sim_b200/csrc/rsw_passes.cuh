@@ -429,12 +429,14 @@ template <int T> struct ColTab {
 // 14.0; 24 warps at 80 registers: 24.3 and 14.0. Rows of 2^13 and more fill
 // the SM at these counts anyway. Shorter rows stay uncapped: the caps made
 // them spill in the factor tables' sincospi (complex128 2^10 2 %, 2^8 7 % and
-// 2^11 forward rows 10 % slower). So do single rows (no chirp form). Radix-32
-// rows of complex64 run 16 warps at 128 registers.
+// 2^11 forward rows 10 % slower). So do per-sample rows (no chirp form), but
+// for complex128 2^12 (a propagation of 2^24 with the exact kernel 819 -> 694
+// us, 2^20 56 -> 44) and complex64 2^13. Radix-32 rows of complex64 run 16
+// warps at 128 registers.
 template <typename Real, int LOG_L2, int E, bool CHIRP> constexpr int row_min_ctas() {
     if (E == 32) return sizeof(Real) == 4 && LOG_L2 >= 10 && LOG_L2 < 14 ? 512 / ((1 << LOG_L2) / 32) : 1;
     if (LOG_L2 < (sizeof(Real) == 8 && E == 16 ? 12 : 11)) return 1;
-    if (!CHIRP && !(sizeof(Real) == 4 && LOG_L2 == 13)) return 1;
+    if (!CHIRP && LOG_L2 != (sizeof(Real) == 4 ? 13 : 12)) return 1;
     constexpr int want = (sizeof(Real) == 8 && E == 16 ? 512 : 1024) / ((1 << LOG_L2) / E);
     return want < 1 ? 1 : want;
 }
