@@ -548,6 +548,15 @@ __global__ void __launch_bounds__(row_threads<LOG_L2, Block<Real, LOG_L2, 1, E>:
         return r * B::T + tp;
     };
 
+    // complex64 rows of 2^13, which 64 registers hold only just, wait before the
+    // loop: inside it the wait costs spills (a row pass of 2^24 145 us, 140 so)
+    constexpr bool WAIT_FIRST = B::LIFT && LOG_L2 == 13 && E == 16;
+    if constexpr (WAIT_FIRST) {
+        B::twiddles_loaded();
+        pass_wait();
+        pass_release();
+        __syncthreads();
+    }
     int parity = 0;
     for (int64_t row = blockIdx.x; row < rows; row += gridDim.x, parity ^= 1) {
         // per-row tables, double-buffered by row parity: the next row fills
@@ -623,7 +632,7 @@ __global__ void __launch_bounds__(row_threads<LOG_L2, Block<Real, LOG_L2, 1, E>:
         // the two parts of the four-step factor of register r
         const auto tw_thread = [&](int r) { return SHORT ? thread_tw : vec[B::first_pos(tp, r) & 63]; };
         const auto tw_register = [&](int r) { return SHORT ? vec[r] : vec[64 + (B::first_pos(tp, r) >> 6)]; };
-        if (row == blockIdx.x) {  // what is above does not depend on the preceding kernel
+        if (!WAIT_FIRST && row == blockIdx.x) {  // what is above does not depend on the preceding kernel
             if constexpr (SHORT && CHIRP && !TABLE) {
                 // the row's chirp table into L1 (two launches before this one
                 // wrote it: a column pass, which waited for it, lies between)
