@@ -29,7 +29,7 @@ template <bool DET, bool BT = false> cudaError_t col_dispatch(const PassArgs &a,
             RSW_COL_CASE16(double, 7)
             RSW_COL_E8(double, 8, 16, 16)
             RSW_COL_CASE_E(double, 9, 8, 8) RSW_COL_CASE_E(double, 10, 4, 4) RSW_COL_CASE_E(double, 11, 4, 4)
-            // 2^12 (tunings only): two columns per CTA, 32-byte row segments
+            // 2^12 (the default at 2^24 and 2^25): two columns per CTA, 32-byte row segments
             RSW_COL_E8(double, 12, 2, 2)
         default: return cudaErrorInvalidValue;
         }

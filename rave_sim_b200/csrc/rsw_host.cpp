@@ -463,11 +463,11 @@ template <typename T> static rsw_status plan_tables(rsw_plan_s *p) {
     return RSW_OK;
 }
 
-// Level split of N = 2^lg: one row level up to the row kernel's limit; two
-// levels (columns x rows) up to the column limit times the row limit; beyond
-// that three levels, N = N1 x Nb x Nr, with rows of the row kernel's maximum
-// length and the rest split evenly between the outer column level and the
-// middle level (both run by the column kernel).
+// Level split of N = 2^lg: one row level up to SINGLE_ROW_MAX (by tuning up to
+// the row kernel's limit); two levels (columns x rows) up to the column limit
+// times the row limit; beyond that three levels, N = N1 x Nb x Nr, with rows of
+// the row kernel's maximum length and the rest divided between the outer column
+// level and the middle level (both run by the column kernel; plan_split).
 // A split from a tuning (levels 1..3): single level; columns of 2^log_rows
 // and rows of the rest; columns, a middle level of 2^log_mid and rows.
 static rsw_status tuned_split(int lg, int dtype, const rsw_tuning &t, int *l1, int *lb, int *lr) {
