@@ -632,14 +632,42 @@ __global__ void __launch_bounds__(row_threads<LOG_L2, Block<Real, LOG_L2, 1, E>:
         // the two parts of the four-step factor of register r
         const auto tw_thread = [&](int r) { return SHORT ? thread_tw : vec[B::first_pos(tp, r) & 63]; };
         const auto tw_register = [&](int r) { return SHORT ? vec[r] : vec[64 + (B::first_pos(tp, r) >> 6)]; };
+        // The row's chirp table (two launches before this one wrote it: a column
+        // pass, which waited for it, lies between). complex128 rows of few warps
+        // take their entries to registers, all loads in flight at once (loaded
+        // where they are used, four at a time, they wait for L2 one batch after
+        // the other). Issued here, and multiplied by the row's factors before
+        // the wait, they cost a short launch nothing: three gratings at 2^16 322
+        // us with the loads behind the wait, 311 so.
+        constexpr bool EARLY = SHORT && CHIRP && !TABLE && !B::LIFT;
+        [[maybe_unused]] Cx h[EARLY ? E : 1];
+        if constexpr (EARLY) {
+            if (a.pr.has_h) {
+                const Cx *h3 = static_cast<const Cx *>(BATCH ? a.bpr[row >> log_m].h3 : a.pr.h3) + tp;
+#pragma unroll
+                for (int r = 0; r < E; ++r) h[r] = __ldg(h3 + r * B::T);
+            }
+        }
+        // ... and their products with the row's factors, the first row's before the wait
+        [[maybe_unused]] const auto fold_chirp = [&] {
+            if constexpr (EARLY) {
+#pragma unroll
+                for (int r = 0; r < E; ++r) h[r] = cmul(cmul(thread_chirp, chp[RO + r]), h[r]);
+            }
+        };
         if (!WAIT_FIRST && row == blockIdx.x) {  // what is above does not depend on the preceding kernel
-            if constexpr (SHORT && CHIRP && !TABLE) {
-                // the row's chirp table into L1 (two launches before this one
-                // wrote it: a column pass, which waited for it, lies between)
+            if constexpr (SHORT && CHIRP && !TABLE && !EARLY) {
+                // complex64: into L1
                 if (a.pr.has_h) {
                     const char *h3 = static_cast<const char *>(BATCH ? a.bpr[row >> log_m].h3 : a.pr.h3);
                     for (int k = tp; k < L / 8; k += B::NT)
                         asm volatile("prefetch.global.L1 [%0];" ::"l"(h3 + k * 128));
+                }
+            }
+            if constexpr (EARLY) {
+                if (a.pr.has_h) {
+                    __syncthreads();  // chp is complete
+                    fold_chirp();
                 }
             }
             B::twiddles_loaded();
@@ -666,19 +694,6 @@ __global__ void __launch_bounds__(row_threads<LOG_L2, Block<Real, LOG_L2, 1, E>:
             }
         };
         Cx v[E];
-        // complex128 rows of few warps: the chirp table's entries in flight with
-        // the samples, all at once (loaded where they are used, four at a time,
-        // they wait for L2 one batch after the other: the split steps of a
-        // simulation at 2^16 450 against 437 us)
-        constexpr bool EARLY = SHORT && CHIRP && !TABLE && !B::LIFT;
-        [[maybe_unused]] Cx h[EARLY ? E : 1];
-        if constexpr (EARLY) {
-            if (a.pr.has_h) {
-                const Cx *h3 = static_cast<const Cx *>(BATCH ? a.bpr[row >> log_m].h3 : a.pr.h3) + tp;
-#pragma unroll
-                for (int r = 0; r < E; ++r) h[r] = __ldg(h3 + r * B::T);
-            }
-        }
         if (!(flags & PF_SPEC_IN)) {
 #pragma unroll
             for (int r = 0; r < E; ++r) v[r] = (flags & PF_ONES) ? one_c<Cx>() : __ldcg(gin + B::first_pos(tp, r));
@@ -760,10 +775,11 @@ __global__ void __launch_bounds__(row_threads<LOG_L2, Block<Real, LOG_L2, 1, E>:
                     if (cut_span == 0) rotate(std::false_type{});
                     else rotate(std::true_type{});
                 } else if constexpr (SHORT) {
+                if (row != blockIdx.x) fold_chirp();
                 const auto multiply = [&](auto cut) {
 #pragma unroll
                     for (int r = 0; r < E; ++r) {
-                        const Cx x = cmul(v[r], cmul(cmul(thread_chirp, chp[RO + r]), h[r]));
+                        const Cx x = cmul(v[r], h[r]);
                         v[r] = decltype(cut)::value ? zero_cut(r, x) : x;
                     }
                 };
