@@ -473,7 +473,13 @@ template <int LOG_L2, int NT, bool CHIRP> constexpr int row_threads() {
 // that it takes the long rows' register caps: in the per-sample kernel, which
 // needs 220 to 254 registers, the Bluestein rows ran 8 warps on an SM (2^11
 // complex64, 2^22 samples: 46 us).
-template <typename Real, int LOG_L2, int E, bool CHIRP, bool TWF = false, bool BATCH = false, bool TABLE = false>
+// SINGLE: single-level plans (per-sample form), without the code of the levels
+// around the row: a launch of one short row waits for its instructions most of
+// the time (8 to 10 of 12 cycles per instruction). A simulation of 2^10
+// complex128 samples with gratings and a sample 484 -> 384 us, 2^11 gratings
+// 295 -> 248.
+template <typename Real, int LOG_L2, int E, bool CHIRP, bool TWF = false, bool BATCH = false, bool TABLE = false,
+          bool SINGLE = false>
 __global__ void __launch_bounds__(row_threads<LOG_L2, Block<Real, LOG_L2, 1, E>::NT, CHIRP>(),
                                   row_min_ctas<Real, LOG_L2, E, CHIRP>()) row_pass_kernel(PassArgs a) {
     using B = Block<Real, LOG_L2, 1, E>;
@@ -489,16 +495,19 @@ __global__ void __launch_bounds__(row_threads<LOG_L2, Block<Real, LOG_L2, 1, E>:
     Tw *tw = reinterpret_cast<Tw *>(smraw + B::DATA);
     Lf *const tabs = reinterpret_cast<Lf *>(smraw + (B::SMEM + 15) / 16 * 16);
     const int tp = threadIdx.x;
-    const int flags = a.flags;
+    const int flags = SINGLE ? a.flags & ~(PF_TW | PF_TWF) : a.flags;
     const int64_t rows = a.n >> LOG_L2;
-    const int log_m = a.log_n1 + a.log_nb;  // spectrum index k = kbase + 2^log_m * k2
+    const int log_n1 = SINGLE ? 0 : a.log_n1, log_nb = SINGLE ? 0 : a.log_nb;
+    const int log_m = log_n1 + log_nb;  // spectrum index k = kbase + 2^log_m * k2
     // row -> (p1, pb): spectrum index base kbase = k1 + N1 kb (rows beyond one
     // transform belong to the next one of a batch)
     const auto row_k1 = [&](int64_t row) {
-        return digitrev_w((row >> a.log_nb) & ((int64_t(1) << a.log_n1) - 1), a.log_n1, a.rb_n1);
+        return SINGLE ? 0 : digitrev_w((row >> log_nb) & ((int64_t(1) << log_n1) - 1), log_n1, a.rb_n1);
     };
-    const auto row_kb = [&](int64_t row) { return digitrev_w(row & ((int64_t(1) << a.log_nb) - 1), a.log_nb, a.rb_nb); };
-    const auto row_k = [&](int64_t row) { return row_k1(row) + (row_kb(row) << a.log_n1); };
+    const auto row_kb = [&](int64_t row) {
+        return SINGLE ? 0 : digitrev_w(row & ((int64_t(1) << log_nb) - 1), log_nb, a.rb_nb);
+    };
+    const auto row_k = [&](int64_t row) { return row_k1(row) + (row_kb(row) << log_n1); };
     constexpr int HT = row_threads<LOG_L2, B::NT, CHIRP>();
     if (HT == B::NT || tp < B::NT) B::load_twiddles(tw, static_cast<const Tw *>(a.tw_row));
     // the transfer function of the CTA's row (row_threads), register r of thread
@@ -572,8 +581,8 @@ __global__ void __launch_bounds__(row_threads<LOG_L2, Block<Real, LOG_L2, 1, E>:
         [[maybe_unused]] Lf thread_tw{};                                 // SHORT: its four-step factor
         // the conjugate four-step twiddle of the innermost split uses tw_k
         const int64_t k1 = row_k1(row), kb = row_kb(row);
-        const int64_t kbase = k1 + (kb << a.log_n1);
-        const int64_t tw_k = a.log_nb > 0 ? kb : k1;
+        const int64_t kbase = k1 + (kb << log_n1);
+        const int64_t tw_k = log_nb > 0 ? kb : k1;
         if (CHIRP && !TABLE && a.pr.has_h) {
             // phase of the row: G kbase^2 + g1 k2s with g1 = 2 M G kbase (turns),
             // M = 2^log_m; P[a] = A exp(2 pi i (G kbase^2 + g1 a)), Q[b] = exp(2 pi i 64 g1 b).
@@ -1233,10 +1242,10 @@ static inline bool pass_serial(const PassArgs &a, size_t elem) {
     return a.serial || a.n >= (int64_t(1) << 29) / int64_t(elem);
 }
 
-template <typename Real, int LG, int E, bool CH, bool TWF, bool BT, bool TABLE = false>
+template <typename Real, int LG, int E, bool CH, bool TWF, bool BT, bool TABLE = false, bool SINGLE = false>
 static cudaError_t row_launch(const PassArgs &a, cudaStream_t s) {
     using B = Block<Real, LG, 1, E>;
-    auto k = row_pass_kernel<Real, LG, E, CH, TWF, BT, TABLE>;
+    auto k = row_pass_kernel<Real, LG, E, CH, TWF, BT, TABLE, SINGLE>;
     const size_t smem = (B::SMEM + 15) / 16 * 16 + 2 * size_t(RowTab<LG, E>::NV + RowTab<LG, E>::NCH) * 16;
     // the row's transfer function in shared memory (row_threads)
     constexpr int HT = row_threads<LG, B::NT, CH>();
@@ -1268,11 +1277,15 @@ static cudaError_t row_impl(const PassArgs &a, cudaStream_t s) {
     if constexpr (BT && !CH) {
         return cudaErrorInvalidValue;
     } else {
+        if constexpr (!CH) {
+            if (a.log_n1 == 0) return row_launch<Real, LG, E, CH, false, BT, false, true>(a, s);
+        }
         if constexpr (LG >= 7) {
             if (a.flags & PF_TWF) return row_launch<Real, LG, E, CH, true, BT>(a, s);
         }
         if (a.flags & PF_TWF) return cudaErrorInvalidValue;
-        return row_launch<Real, LG, E, CH, false, BT>(a, s);
+        if constexpr (CH || LG >= 7) return row_launch<Real, LG, E, CH, false, BT>(a, s);
+        else return cudaErrorInvalidValue;
     }
 }
 
