@@ -418,7 +418,8 @@ struct Block : Radix<LOG_L, E_, direct_max_ls(2 * sizeof(Real), LOG_L, digit_bit
     // their 7 direct lookups for products. A running product W^(j(q-1)) W^j
     // needs one lookup only, but multiplies that entry's rounding by q: an rms
     // error of 4.9e-16 per radix-16 factor and 2.5e-16 per radix-8 one, against
-    // 0.9e-16 and 1.2e-16. complex64 keeps the lookups.
+    // 0.9e-16 and 1.2e-16. Same times at 2^20 to 2^24; rows of 2^13 pay 2 % for it
+    // (a propagation of 2^25 1177 -> 1200 us). complex64 keeps the lookups.
     template <int s> static constexpr bool by_powers() {
         return sizeof(Real) == 8 && (!Rx::direct(s) || (E == 8 && LOG_L >= 10));
     }
